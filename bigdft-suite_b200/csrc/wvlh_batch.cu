@@ -143,8 +143,8 @@ extern "C" int wvlh_ctx_synchronize(wvlh_ctx *ctx)
 namespace wvlh {
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no link
 // against the driver library)
-bool encode_tile_map(CUtensorMap *map, const void *base, int elem_bytes, long long W, long long H, long long Z,
-                     long long norb, long long orb_stride_elems)
+bool encode_tile_map(CUtensorMap *map, const void *base, int elem_bytes, long long W, long long pitch, long long H,
+                     long long Z, long long norb, long long orb_stride_elems)
 {
     static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
     static bool looked = false;
@@ -158,7 +158,7 @@ bool encode_tile_map(CUtensorMap *map, const void *base, int elem_bytes, long lo
         cudaGetLastError();
     }
     if (!fn || Z > 256 || Z < 1 || W < 1 || H < 1 || norb < 1) return false;
-    const long long rowb = W * elem_bytes, planeb = rowb * H, orbb = orb_stride_elems * elem_bytes;
+    const long long rowb = pitch * elem_bytes, planeb = rowb * H, orbb = orb_stride_elems * elem_bytes;
     // strides and the base address must be multiples of 16 bytes
     if ((rowb % 16) || (planeb % 16) || (orbb % 16) || ((uintptr_t)base % 16)) return false;
     const cuuint64_t dim[4] = {(cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)Z, (cuuint64_t)norb};
@@ -173,31 +173,24 @@ bool encode_tile_map(CUtensorMap *map, const void *base, int elem_bytes, long lo
 }
 }  // namespace wvlh
 
-// Validate the reference's 1-based keys of one region and decode them into
-// {i0, i2, len, jj0} plus per-plane segment ranges (wavelib/un-compress.f90:896-905).
-static int decode_keys(const int *N, int nseg, const int32_t *keyg, const int32_t *keyv, std::vector<int4> &seg,
-                       std::vector<int> &plane, int &nvctr)
+// Validate the reference's 1-based keys of one region and find the cells of
+// each z-plane: plane[i3] is the compressed index of the first cell at or after
+// plane i3 (wavelib/un-compress.f90:896-905).
+static int decode_keys(const int *N, int nseg, const int32_t *keyg, const int32_t *keyv, std::vector<int> &plane, int &nvctr)
 {
     const long long n12 = (long long)N[0] * N[1];
     if (nseg > 0 && (!keyg || !keyv)) return WVLH_ERR_ARG;
     if (check_keys(N, nseg, keyg, keyv, nullptr)) return WVLH_ERR_KEYS;
-    seg.resize(nseg);
-    plane.assign(N[2] + 1, nseg);
+    plane.assign(N[2] + 1, 0);
     long long cum = 0;
     int cur_plane = 0;
     for (int s = 0; s < nseg; ++s) {
         const long long j0 = keyg[2 * s], j1 = keyg[2 * s + 1];
-        long long ii = j0 - 1;
-        const int i3 = (int)(ii / n12);
-        ii -= (long long)i3 * n12;
-        const int i2 = (int)(ii / N[0]);
-        const int i0 = (int)(ii - (long long)i2 * N[0]);
-        const int len = (int)(j1 - j0 + 1);
-        seg[s] = make_int4(i0, i2, len, (int)cum);
-        while (cur_plane <= i3) plane[cur_plane++] = s;
-        cum += len;
+        const int i3 = (int)((j0 - 1) / n12);
+        while (cur_plane <= i3) plane[cur_plane++] = (int)cum;
+        cum += j1 - j0 + 1;
     }
-    while (cur_plane <= N[2]) plane[cur_plane++] = nseg;
+    while (cur_plane <= N[2]) plane[cur_plane++] = (int)cum;
     nvctr = (int)cum;
     return WVLH_OK;
 }
@@ -222,11 +215,10 @@ static int region_make(int device, const wvlh_locreg &L, wvlh_region **out)
         if (L.periodic[k] && L.n[k] < 8) return WVLH_ERR_ARG;
     }
     if (L.nseg_c < 0 || L.nseg_f < 0) return WVLH_ERR_ARG;
-    std::vector<int4> sc, sf;
     std::vector<int> pc, pf;
     int nvc = 0, nvf = 0, rc;
-    if ((rc = decode_keys(L.n, L.nseg_c, L.keyg_c, L.keyv_c, sc, pc, nvc))) return rc;
-    if ((rc = decode_keys(L.n, L.nseg_f, L.keyg_f, L.keyv_f, sf, pf, nvf))) return rc;
+    if ((rc = decode_keys(L.n, L.nseg_c, L.keyg_c, L.keyv_c, pc, nvc))) return rc;
+    if ((rc = decode_keys(L.n, L.nseg_f, L.keyg_f, L.keyv_f, pf, nvf))) return rc;
     wvlh_region *r = new wvlh_region();
     r->device = device;
     LrDev &d = r->lr;
@@ -243,15 +235,15 @@ static int region_make(int device, const wvlh_locreg &L, wvlh_region **out)
     std::vector<uint32_t> kgc(L.keyg_c, L.keyg_c + 2 * (size_t)L.nseg_c), kvc(L.keyv_c, L.keyv_c + L.nseg_c);
     std::vector<uint32_t> kgf(L.keyg_f, L.keyg_f + 2 * (size_t)L.nseg_f), kvf(L.keyv_f, L.keyv_f + L.nseg_f);
     Packer pk;
-    pk.add(sc, &d.seg_c);
-    pk.add(sf, &d.seg_f);
     pk.add(pc, &d.plane_c);
     pk.add(pf, &d.plane_f);
     pk.add(kgc, &r->keyg_c);
     pk.add(kvc, &r->keyv_c);
     pk.add(kgf, &r->keyg_f);
     pk.add(kvf, &r->keyv_f);
-    if (cudaMalloc(&r->mem, pk.img.size()) != cudaSuccess) {
+    // the cell tables follow the uploaded block and are expanded on the device
+    const size_t tab = (pk.img.size() + 255) & ~size_t(255);
+    if (cudaMalloc(&r->mem, tab + sizeof(int) * ((size_t)nvc + nvf)) != cudaSuccess) {
         r->mem = nullptr;
         region_free(r);
         return WVLH_ERR_NOMEM;
@@ -261,6 +253,21 @@ static int region_make(int device, const wvlh_locreg &L, wvlh_region **out)
         return WVLH_ERR_CUDA;
     }
     pk.place(r->mem);
+    int *pos = reinterpret_cast<int *>(static_cast<unsigned char *>(r->mem) + tab);
+    d.pos_c = pos;
+    d.pos_f = pos + nvc;
+    const int pitch = plane_pitch(d.N[0], d.per[0]);
+    if (L.nseg_c)
+        k_cell_places<<<(L.nseg_c + 7) / 8, 256>>>(d.N[0], d.N[1], pitch, L.nseg_c, (const int32_t *)r->keyg_c,
+                                                   (const int32_t *)r->keyv_c, pos);
+    if (L.nseg_f)
+        k_cell_places<<<(L.nseg_f + 7) / 8, 256>>>(d.N[0], d.N[1], pitch, L.nseg_f, (const int32_t *)r->keyg_f,
+                                                   (const int32_t *)r->keyv_f, pos + nvc);
+    // launches may follow on any stream
+    if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(0) != cudaSuccess) {
+        region_free(r);
+        return WVLH_ERR_CUDA;
+    }
     *out = r;
     return WVLH_OK;
 }
@@ -292,14 +299,8 @@ extern "C" int64_t wvlh_region_grid_size(const wvlh_region *r)
     return n;
 }
 
-// scratch elements of one orbital of a region in the fused kernels (P, Q, Z)
-static long long orbital_scratch(const LrDev &d)
-{
-    const int G3 = 2 * d.N[2];
-    const int F1 = fine_len(d.N[0], d.per[0]), F2 = fine_len(d.N[1], d.per[1]);
-    const int I1 = isf_len(d.N[0], d.per[0]), I2 = isf_len(d.N[1], d.per[1]);
-    return (long long)G3 * F2 * F1 * 2 + (long long)G3 * I2 * I1;
-}
+// scratch elements of one orbital of a region in the fused kernels
+static long long orbital_scratch(const LrDev &d) { return orb_scratch(d.N, d.per).total; }
 
 extern "C" int64_t wvlh_region_scratch_bytes(const wvlh_region *r, int precision)
 {
@@ -331,7 +332,7 @@ static void layout(wvlh_batch *b, const std::vector<int> &orb_lr, const std::vec
     std::vector<long long> orb_off;
     long long psi_off = 0, scr = 0;
     int stride = 0;
-    size_t planeA = 0, planeB = 0, sm2_elems = 0;
+    size_t planeA = 0, planeB = 0, sm2_elems = 0, z0_elems = 0, z1_elems = 0;
     std::vector<PlaneShape> shapes32, shapes64;  // plane geometry per orbital (CTA-size choice)
     b->pot_off.assign(pot_key.begin(), pot_key.end());
     for (int o = 0; o < norb; ++o) {
@@ -346,12 +347,11 @@ static void layout(wvlh_batch *b, const std::vector<int> &orb_lr, const std::vec
         q.pad = 0;
         q.psi = psi_off;
         q.pot = pot_key[o];
+        const OrbScratch sc = orb_scratch(d.N, d.per);
         q.sP = scr;
-        scr += (long long)G3 * F2 * F1;
-        q.sQ = scr;
-        scr += (long long)G3 * I2 * I1;
-        q.sZ = scr;
-        scr += (long long)G3 * F2 * F1;
+        q.sZ = scr + sc.z;
+        q.sQ = scr + sc.q;
+        scr += (sc.total + 3) & ~3LL;   // orbitals start on 16 bytes (TMA strides)
         q.c = 0.0;
         q.in_ptr = abs ? abs[o].psi : nullptr;
         q.out_ptr = abs ? abs[o].hpsi : nullptr;
@@ -363,21 +363,18 @@ static void layout(wvlh_batch *b, const std::vector<int> &orb_lr, const std::vec
         orb_len.push_back(len);
         psi_off += len;
         const int ntx0 = (I1 + TX_ - 1) / TX_, nty0 = (I2 + TY_ - 1) / TY_;
-        const int ntx1 = (F1 + TX_ - 1) / TX_, nty1 = (F2 + TY_ - 1) / TY_;
+        const int ntx1 = (2 * N1 + TX_ - 1) / TX_, nty1 = (2 * N2 + TY_ - 1) / TY_;
         pre13.push_back(pre13.back() + G3);
         pre2.push_back(pre2.back() + ntx0 * nty0);
         pre2p.push_back(pre2p.back() + ntx1 * nty1);
         stride = std::max(stride, std::max(ntx0 * nty0, ntx1 * nty1 + G3));
-        // plane buffer A: rows (y) x pitch (x); B holds P (F2 rows x pitch)
-        // or a transposed plane (lines along x, each at the vec_pitch of its
-        // y length).  Coarse lines are stored with the wavelet half at an
-        // even offset (coarse_width).
+        // plane buffer A: rows (y) x pitch (x), a real-space or a wavelet
+        // plane (a row's wavelet half at an even offset, coarse_width); B: the
+        // 2 N2 rows of a wavelet plane or of one with real-space rows
         const int W1 = coarse_width(N1), W2 = coarse_width(N2);
-        const int pitch = vec_pitch(std::max(W1, std::max(F1, I1)));
+        const int pitch = plane_pitch(N1, d.per[0]);
         const int rows = std::max(W2, std::max(F2, I2));
-        const long long bT = std::max(std::max((long long)F1 * vec_pitch(W2), (long long)I1 * vec_pitch(F2)),
-                                      std::max((long long)F1 * vec_pitch(I2), (long long)W1 * vec_pitch(F2)));
-        const long long bsz = std::max((long long)F2 * pitch, bT);
+        const long long bsz = 2LL * N2 * pitch;
         planeA = std::max(planeA, (size_t)rows * pitch);
         {
             const long long len = std::max(W1, std::max(F1, I1)), w = (long long)G3 * rows * pitch;
@@ -388,6 +385,8 @@ static void layout(wvlh_batch *b, const std::vector<int> &orb_lr, const std::vec
         planeB = std::max(planeB, (size_t)bsz);
         const int zl = std::max(G3, std::max(F3, I3));
         sm2_elems = std::max(sm2_elems, (size_t)2 * zl * TX_ * TY_);
+        z0_elems = std::max(z0_elems, (size_t)(G3 + I3) * TX_ * TY_);
+        z1_elems = std::max(z1_elems, (size_t)G3 * TX_ * TY_);
     }
     p.psi_total = psi_off;
     p.all_periodic = true;
@@ -399,11 +398,10 @@ static void layout(wvlh_batch *b, const std::vector<int> &orb_lr, const std::vec
         for (int o = 1; o < norb && one; ++o) one = orb_lr[o] == orb_lr[0];
         if (one) {
             const LrDev &d = lrd[orb_lr[0]];
-            const long long G3 = 2LL * d.N[2], F1 = fine_len(d.N[0], d.per[0]), F2 = fine_len(d.N[1], d.per[1]),
-                            I1 = isf_len(d.N[0], d.per[0]), I2 = isf_len(d.N[1], d.per[1]);
-            p.orb_scratch = 2 * G3 * F2 * F1 + G3 * I2 * I1;
-            const long long dims[5] = {G3, F1, F2, I1, I2};
-            for (int k = 0; k < 5; ++k) p.tile_dims[k] = dims[k];
+            const OrbScratch sc = orb_scratch(d.N, d.per);
+            p.orb_scratch = (sc.total + 3) & ~3LL;
+            p.tile = TileDims{2LL * d.N[0], 2LL * d.N[1], 2LL * d.N[2], isf_len(d.N[0], d.per[0]),
+                              isf_pitch(d.N[0], d.per[0]), isf_len(d.N[1], d.per[1]), sc.q};
         }
     }
     p.part_stride = stride;
@@ -418,6 +416,10 @@ static void layout(wvlh_batch *b, const std::vector<int> &orb_lr, const std::vec
     p.smem13[1] = (planeA + planeB) * sizeof(double);
     p.smem2[0] = sm2_elems * sizeof(float);
     p.smem2[1] = sm2_elems * sizeof(double);
+    p.smem_z0[0] = z0_elems * sizeof(float);
+    p.smem_z0[1] = z0_elems * sizeof(double);
+    p.smem_z1[0] = z1_elems * sizeof(float);
+    p.smem_z1[1] = z1_elems * sizeof(double);
     p.n_work13 = pre13.back();
     p.n_work2 = pre2.back();
     p.n_work2p = pre2p.back();

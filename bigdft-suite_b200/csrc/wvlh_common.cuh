@@ -72,6 +72,26 @@ constexpr double kMfSeedTap = 0.5;
 __host__ __device__ __forceinline__ int fine_len(int N, int per) { return per ? 2 * N : 2 * N + 14; }
 __host__ __device__ __forceinline__ int isf_len(int N, int per) { return per ? 2 * N : 2 * N + 29; }
 
+// Row pitch of a real-space plane in the fused kernels' scratch: the 2N points
+// of a periodic row, or a free row's 2N + 29 rounded up to 16 bytes of FP32,
+// so that rows start on a point pair and TMA can stride them.
+__host__ __device__ __forceinline__ int isf_pitch(int N, int per) { return per ? 2 * N : (2 * N + 29 + 3) & ~3; }
+
+// Scratch of one orbital in the fused kernels, in elements: D at 0, Z2 at z, Q
+// (then Z1) at q.  The total is the room of three planes stacks on the fine
+// and real-space grids (what callers budget, wvlh_region_scratch_bytes): the
+// two wavelet stacks are smaller than fine ones in free directions, which
+// covers Q's padded rows.
+struct OrbScratch {
+    long long z, q, total;
+};
+__host__ __device__ inline OrbScratch orb_scratch(const int *N, const int *per)
+{
+    const long long G3 = 2LL * N[2], F1 = fine_len(N[0], per[0]), F2 = fine_len(N[1], per[1]);
+    const long long w = G3 * 4 * N[0] * N[1];
+    return OrbScratch{w, 2 * w, 2 * G3 * F1 * F2 + G3 * isf_len(N[0], per[0]) * isf_len(N[1], per[1])};
+}
+
 // Periodic index for -L <= p < 3L, without a division.  The fused passes only
 // see periodic lines of at least 8 coarse / 16 fine points, and their windows
 // reach at most 15 points below and SEG + 13 (<= 21) points above the line.
@@ -93,6 +113,25 @@ __device__ __forceinline__ int wrap_near(int p, int L)
 __host__ __device__ constexpr int half_off(int N) { return (N + 1) & ~1; }
 __host__ __device__ constexpr int coarse_width(int N) { return half_off(N) + N; }
 __host__ __device__ constexpr int vec_pitch(int m) { return ((m + 1) & ~1) + ((((m + 1) & ~1) & 3) == 0 ? 2 : 0); }
+
+// row pitch of the plane kernels' buffers for a box of N1 coarse cells in x
+__host__ __device__ __forceinline__ int plane_pitch(int N1, int per1)
+{
+    const int w = 2 * half_off(N1), f = fine_len(N1, per1), r = isf_len(N1, per1);
+    const int m = w > f ? w : f;
+    return vec_pitch(m > r ? m : r);
+}
+
+// Cell table of one key set (LrDev::pos_c / pos_f): one warp per segment.
+static __global__ void k_cell_places(int N1, int N2, int pitch, int nseg, const int32_t *__restrict__ keyg,
+                                     const int32_t *__restrict__ keyv, int *__restrict__ pos)
+{
+    const int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (s >= nseg) return;
+    const int i = keyg[2 * s] - 1, len = keyg[2 * s + 1] - i, j = keyv[s] - 1;
+    const int line = i / N1, x = i - line * N1, y = line % N2;
+    for (int t = lane; t < len; t += 32) pos[j + t] = y * pitch + x + t;
+}
 
 template <class T> struct Pair;
 template <> struct Pair<float> { using type = float2; };

@@ -5,29 +5,31 @@
 // The reference applies locham to one orbital at a time as 13 full-array
 // passes (uncompress, 3x syn, 3x MF, xV, 3x MF^T, 3x kinetic, 3x ana,
 // compress: orbitals/daubisf.f90:214-331, locregs/locreg_operations.f90:2502-2937,
-// OpenCL/Hamiltonian.c:105-172).  Because every 1D operator acts on one
-// axis, the chain factorises as
-//     Hpsi = A_x A_y [ Mt_x Mt_y Z1 + Z2 + (K_x + K_y) P ]
-//     P  = S_x S_y psi,    Q = M_x M_y P                       (plane kernel K1)
-//     Z1 = A_z Mt_z V M_z S_z Q,   Z2 = A_z K_z S_z P            (z kernel K2)
-// (S syn, A ana, M magic filter, K kinetic) so that each kernel keeps a whole
-// xy-plane or a whole z-pencil tile in shared memory and chains its 1D passes
-// there.  E_pot = sum V r^2 comes from K2; E_kin = sum_d <X|K_d X> with
-// X = S^3 psi: the z part from K2 on X itself, the x,y parts from K3 on P
-// (<X|K_x X> = <P|K_x P> because S_z is an isometry).  Energies are reduced
-// in FP64 into per-CTA partial slots and summed in a fixed order.
+// OpenCL/Hamiltonian.c:105-172).  Every 1D operator acts on one axis, and
+// synthesis is an isometry per axis with analysis its transpose, so the chain is
+//     Hpsi = B^T_x B^T_y B^T_z V B_z B_y B_x psi + (T_x + T_y + T_z) psi
+//     B = M S (synthesis, then magic filter), T = A K S (the kinetic operator
+//     in the wavelet basis), each one composed pass (wvlh_lines.cuh):
+//     D = psi's wavelet plane, Q = B_y B_x D                  (plane kernel K1)
+//     Z1 = B^T_z (V . B_z Q) in place of Q, Z2 = T_z D          (z kernel K2)
+//     Hpsi = B^T_x B^T_y Z1 + (T_x + T_y) D + Z2              (plane kernel K3)
+// so that each kernel keeps a whole xy-plane or a whole z-pencil tile in
+// shared memory.  E_pot = sum V r^2 comes from K2; E_kin = <psi | T psi>, its
+// z part from K2, the x and y parts from K3.  Energies are reduced in FP64
+// into per-CTA partial slots and summed in a fixed order.
 //
 // The same kernels in MODE_LOCDEN give the density rho += hfac (M^3 S^3 psi)^2
 // (OpenCL/Density.c:37-55, sumrho.f90:472-577) through K1 (Q only) and a
 // z-kernel that loops over the orbitals sharing a density grid, and in
 // MODE_PRECOND the preconditioner operator D^-1/2 A (c + T) S D^-1/2 of
-// OpenCL/Preconditioner.c:98-128 through K1 (scaled gather, P only), the
-// kinetic chain of K2 and K3 (Z2 + c P + (K_x+K_y) P, scaled scatter).
+// OpenCL/Preconditioner.c:98-128, which is D^-1/2 (c + T_x + T_y + T_z) D^-1/2
+// in the wavelet basis, through K1 (scaled gather, D only), T_z of K2 and K3
+// (Z2 + c D + (T_x + T_y) D, scaled scatter).
 //
 // This file is the implementation shared by the translation units
-// wvlh_fused_f32.cu and wvlh_fused_f64.cu, which instantiate the launchers of
-// one precision each (the two compile in parallel); the common out-of-line
-// helpers are compiled in the FP64 unit (WVLH_FUSED_COMMON).
+// wvlh_{locham,locden,precond}_{f32,f64}.cu, each of which instantiates one
+// launcher in one precision (they compile in parallel); the common out-of-line
+// helpers are compiled in one of them (WVLH_FUSED_COMMON).
 #pragma once
 #include <cuda_runtime.h>
 
@@ -36,7 +38,7 @@
 
 #include "wvlh_common.cuh"
 #include "wvlh_internal.h"
-#include "wvlh_pairs.cuh"
+#include "wvlh_lines.cuh"
 #include "wvlh_tma.cuh"
 
 namespace wvlh {
@@ -50,14 +52,20 @@ constexpr int TC = TX * TY;
 constexpr int kZAlign = 128;
 constexpr int kZExtra = 32 * 8 + 16;
 
-template <class T> struct Seg;
-template <> struct Seg<float> { static constexpr int v = 8; };
-template <> struct Seg<double> { static constexpr int v = 4; };
+// coarse points of one thread's segment, all passes and both precisions: six
+// give the 48-point lines of a 96 x 96 plane two full rounds of 384 threads
+// (rows) and one (columns), and a 32-column tile one round of 256
+constexpr int kSeg = 6;
 
+// A wavelet line holds N scaling and N wavelet coefficients.  In global memory
+// a wavelet plane is dense, G2 = 2 N2 rows of G1 = 2 N1 points.  In shared
+// memory the wavelet half of a row starts at the even offset H1 (rows move as
+// point pairs), the rows stay dense: row y of the wavelet half at N2 + y.
 struct Dims {
     int N1, N2, N3, p1, p2, p3;
-    int H1, H2;  // offsets of the wavelet halves of the coarse x and y lines
-    int G1, G2, G3, F1, F2, F3, I1, I2, I3;
+    int H1;               // offset of the wavelet half of a row in shared memory
+    int G1, G2, G3, I1, I2, I3;
+    int IP1;              // row pitch of the real-space planes Q / Z1 in scratch
     // allper: the batch is known to be periodic in every direction, which lets
     // the compiler drop the free-boundary variants from the kernel
     __device__ __forceinline__ Dims(const LrDev &L, bool allper)
@@ -66,34 +74,16 @@ struct Dims {
         p1 = allper ? 1 : L.per[0];
         p2 = allper ? 1 : L.per[1];
         p3 = allper ? 1 : L.per[2];
-        H1 = half_off(N1); H2 = half_off(N2);
-        G1 = coarse_width(N1); G2 = coarse_width(N2); G3 = 2 * N3;
-        F1 = fine_len(N1, p1); F2 = fine_len(N2, p2); F3 = fine_len(N3, p3);
+        H1 = half_off(N1);
+        G1 = 2 * N1; G2 = 2 * N2; G3 = 2 * N3;
         I1 = isf_len(N1, p1); I2 = isf_len(N2, p2); I3 = isf_len(N3, p3);
+        IP1 = isf_pitch(N1, p1);
     }
-    // plane buffer A: rows() lines (y) of pitch() points (x).  The second
-    // buffer B holds P (F2 rows of pitch()) or a transposed plane: the lines
-    // along x of a pass, each of the y length `len` of its plane, at pitch
-    // pitchT(len) — sized per pass, so B is no larger than its largest use.
-    __device__ __forceinline__ int pitch() const { return vec_pitch(max(G1, max(F1, I1))); }
-    __device__ __forceinline__ int rows() const { return max(G2, max(F2, I2)); }
-    __device__ __forceinline__ static int pitchT(int len) { return vec_pitch(len); }
+    // row pitch of the plane buffers A and B; A holds a real-space plane (I2
+    // rows) or a wavelet plane (G2 rows), B G2 rows
+    __device__ __forceinline__ int pitch() const { return plane_pitch(N1, p1); }
+    __device__ __forceinline__ int rows() const { return max(G2, I2); }
 };
-
-__device__ __forceinline__ LineGeom rows_geom(int nrows, int pitch)
-{
-    return LineGeom{nrows, pitch, 1, pitch, 1};
-}
-__device__ __forceinline__ LineGeom cols_geom(int ncols, int pitch)
-{
-    return LineGeom{ncols, 1, pitch, 1, pitch};
-}
-// lines read with unit stride, output written transposed: point q of line l
-// goes to dst[q * dst_pitch + l], so the next pass again reads unit stride
-__device__ __forceinline__ LineGeom xpose_geom(int nlines, int src_pitch, int dst_pitch)
-{
-    return LineGeom{nlines, src_pitch, 1, 1, dst_pitch};
-}
 
 // fine component c=1..7 of psi_f -> (s1,s2,s3) bits (wavelib/un-compress.f90:930-936)
 __device__ __forceinline__ int fs1(int c) { return c & 1; }
@@ -112,35 +102,48 @@ __device__ __forceinline__ double prec_scal(const LrDev &L, double c, int k)
     return 1.0 / sqrt(s);
 }
 
-// Scatter the compressed coefficients of wavelet-basis plane kz into the
-// (G2 x G1, pitch) buffer A, which must be zero.  Wavelet components sit at
-// x + half_off(N1) and y + half_off(N2).  psi points at [psi_c|psi_f]; sc (8
-// factors) scales each component when non-null.
+// The cells of a wavelet z-plane are consecutive in the compressed vector, and
+// each has its place in the shared plane in the region's cell table, so
+// gathering and scattering walk cells with all lanes busy, no segment in
+// sight.  (A warp per segment left a third of the lanes of 48-cell rows idle
+// and cost the plane kernels 45 to 50 instructions a point, more than one of
+// their filter passes.)  A fine cell holds the seven components c = s1 + 2 s2 +
+// 4 s3; a plane takes those of its own s3: the three after the coarse
+// coefficient (s3 = 0) or four (s3 = 1).
+
+// value c (its s1, s2 bits) of a cell sits this far from the cell's place
+__device__ __forceinline__ int comp_ofs(int c, int H1, int wrow) { return fs1(c) * H1 + fs2(c) * wrow; }
+
+struct PlaneCells {
+    int a_c, b_c, a_f, b_f;   // the plane's coarse cells (none when s3 = 1), fine cells
+    int H1, wrow;             // offsets of the x and y wavelet halves in the shared plane
+    __device__ __forceinline__ PlaneCells(const LrDev &L, int pitch, int i3, bool coarse)
+    {
+        a_c = coarse ? L.plane_c[i3] : 0;
+        b_c = coarse ? L.plane_c[i3 + 1] : 0;
+        a_f = L.plane_f[i3];
+        b_f = L.plane_f[i3 + 1];
+        H1 = half_off(L.N[0]);
+        wrow = L.N[1] * pitch;
+    }
+};
+
+// Scatter the compressed coefficients of wavelet plane kz into buffer A, which
+// must be zero.  psi points at [psi_c|psi_f]; sc (8 factors) scales each
+// component when non-null.
 template <class T, class TI, int S3>
 __device__ __forceinline__ void gather_plane_s(T *A, int pitch, const LrDev &L, int i3, const TI *psi, const T *sc)
 {
-    const int H1 = half_off(L.N[0]), H2 = half_off(L.N[1]);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    if (!S3) {
-        const T s0 = sc ? sc[0] : T(1);
-        const int a = L.plane_c[i3], b = L.plane_c[i3 + 1];
-        for (int sg = a + warp; sg < b; sg += nw) {
-            const int4 d = L.seg_c[sg];
-            for (int t = lane; t < d.z; t += 32) A[d.y * pitch + d.x + t] = (T)psi[d.w + t] * s0;
-        }
-    }
+    const PlaneCells p(L, pitch, i3, !S3);
+    const T s0 = sc ? sc[0] : T(1);
+    for (int j = p.a_c + threadIdx.x; j < p.b_c; j += blockDim.x) A[L.pos_c[j]] = (T)psi[j] * s0;
     const TI *pf = psi + L.nvctr_c;
-    const int a = L.plane_f[i3], b = L.plane_f[i3 + 1];
-    for (int sg = a + warp; sg < b; sg += nw) {
-        const int4 d = L.seg_f[sg];
-        for (int t = lane; t < d.z; t += 32) {
-            const TI *src = pf + 7 * (size_t)(d.w + t);
+    for (int j = p.a_f + threadIdx.x; j < p.b_f; j += blockDim.x) {
+        T *a = A + L.pos_f[j];
+        const TI *src = pf + 7 * (size_t)j;
 #pragma unroll
-            for (int c = 1; c <= 7; ++c) {
-                if (fs3(c) != S3) continue;
-                A[(fs2(c) * H2 + d.y) * pitch + fs1(c) * H1 + d.x + t] = (T)src[c - 1] * (sc ? sc[c] : T(1));
-            }
-        }
+        for (int c = 1; c <= 7; ++c)
+            if (fs3(c) == S3) a[comp_ofs(c, p.H1, p.wrow)] = (T)src[c - 1] * (sc ? sc[c] : T(1));
     }
 }
 
@@ -158,32 +161,23 @@ template <class T, class TO, int S3>
 __device__ __forceinline__ void scatter_plane_s(const T *A, int pitch, const LrDev &L, int i3, TO *out, bool accumulate,
                                                 const T *sc)
 {
-    const int H1 = half_off(L.N[0]), H2 = half_off(L.N[1]);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    if (!S3) {
-        const T s0 = sc ? sc[0] : T(1);
-        const int a = L.plane_c[i3], b = L.plane_c[i3 + 1];
-        for (int sg = a + warp; sg < b; sg += nw) {
-            const int4 d = L.seg_c[sg];
-            for (int t = lane; t < d.z; t += 32) {
-                const TO v = (TO)(A[d.y * pitch + d.x + t] * s0);
-                out[d.w + t] = accumulate ? out[d.w + t] + v : v;
-            }
-        }
+    const PlaneCells p(L, pitch, i3, !S3);
+    const T s0 = sc ? sc[0] : T(1);
+#pragma unroll 2
+    for (int j = p.a_c + threadIdx.x; j < p.b_c; j += blockDim.x) {
+        const TO v = (TO)(A[L.pos_c[j]] * s0);
+        out[j] = accumulate ? out[j] + v : v;
     }
     TO *pf = out + L.nvctr_c;
-    const int a = L.plane_f[i3], b = L.plane_f[i3 + 1];
-    for (int sg = a + warp; sg < b; sg += nw) {
-        const int4 d = L.seg_f[sg];
-        for (int t = lane; t < d.z; t += 32) {
-            const size_t i = 7 * (size_t)(d.w + t);
-            TO *dst = pf + i;
+#pragma unroll 2
+    for (int j = p.a_f + threadIdx.x; j < p.b_f; j += blockDim.x) {
+        const T *a = A + L.pos_f[j];
+        TO *dst = pf + 7 * (size_t)j;
 #pragma unroll
-            for (int c = 1; c <= 7; ++c) {
-                if (fs3(c) != S3) continue;
-                const TO v = (TO)(A[(fs2(c) * H2 + d.y) * pitch + fs1(c) * H1 + d.x + t] * (sc ? sc[c] : T(1)));
-                dst[c - 1] = accumulate ? dst[c - 1] + v : v;
-            }
+        for (int c = 1; c <= 7; ++c) {
+            if (fs3(c) != S3) continue;
+            const TO v = (TO)(a[comp_ofs(c, p.H1, p.wrow)] * (sc ? sc[c] : T(1)));
+            dst[c - 1] = accumulate ? dst[c - 1] + v : v;
         }
     }
 }
@@ -195,23 +189,39 @@ __device__ void scatter_plane(const T *A, int pitch, const LrDev &L, int kz, TO 
     else scatter_plane_s<T, TO, 0>(A, pitch, L, kz, out, accumulate, sc);
 }
 
-// Rows of `cols` points walked as point pairs: warp w takes rows w, w + nwarps,
-// ...; its lanes take consecutive pairs of the row.  f(r, c), c even.
+// Rows of `cols` points walked as point pairs, every thread on pairs i =
+// threadIdx.x + k * blockDim.x of the plane: f(shared offset r * spitch + c,
+// global offset r * gpitch + c), c even, advanced without a multiplication.
 template <class F>
-__device__ __forceinline__ void for_row_pairs(int rows, int cols, F &&f)
+__device__ __forceinline__ void for_row_pairs(int rows, int cols, int spitch, int gpitch, F &&f)
 {
-    const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    const int np = cols >> 1;
-    for (int r = threadIdx.x >> 5; r < rows; r += nw)
-        for (int j = lane; j < np; j += 32) f(r, 2 * j);
+    const int np = cols >> 1, nt = blockDim.x;
+    int r = threadIdx.x / np, c = threadIdx.x - r * np;
+    const int dr = nt / np, dc = nt - dr * np;
+    int so = r * spitch + 2 * c, go = r * gpitch + 2 * c;
+    const int ds = dr * spitch + 2 * dc, dg = dr * gpitch + 2 * dc;
+    const int ws = spitch - 2 * np, wg = gpitch - 2 * np;   // one row on, from a column past the end
+    const int n = rows * np;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < n; i += nt) {
+        f(so, go);
+        c += dc;
+        so += ds;
+        go += dg;
+        if (c >= np) {
+            c -= np;
+            so += ws;
+            go += wg;
+        }
+    }
 }
 
-// a dense global plane of `cols`-point rows can move as point pairs when cols
-// is even and the plane starts on a pair (the scratch planes do)
+// a global plane with rows `pitch` points apart can move as point pairs when
+// the pitch is even and the plane starts on a pair
 template <class T>
-__device__ __forceinline__ bool pair_rows(int cols, const T *g)
+__device__ __forceinline__ bool pair_rows(int pitch, const T *g)
 {
-    return !(cols & 1) && !(reinterpret_cast<uintptr_t>(g) & (2 * sizeof(T) - 1));
+    return !(pitch & 1) && !(reinterpret_cast<uintptr_t>(g) & (2 * sizeof(T) - 1));
 }
 
 template <class T>
@@ -226,25 +236,22 @@ __device__ __forceinline__ void zero_region(T *A, int rows, int pitch)
     for (int i = threadIdx.x; i < (rows * pitch) >> 1; i += blockDim.x) a[i] = z;
 }
 
+// column of a dense wavelet row -> its place in a shared-memory row
+__device__ __forceinline__ int wcol(const Dims &d, int c) { return c < d.N1 ? c : c - d.N1 + d.H1; }
+
+// the dense global wavelet plane of shared buffer A (its rows start on pairs:
+// G1 is even and so are the scratch offsets)
 template <class T>
-__device__ __forceinline__ void store_plane(const T *A, int pitch, int rows, int cols, T *g)
+__device__ __forceinline__ void store_wavelet(const T *A, int pitch, const Dims &d, T *g)
 {
-    if (pair_rows(cols, g)) {
-        using V = typename Pair<T>::type;
-        for_row_pairs(rows, cols, [&](int r, int c) {
-            *reinterpret_cast<V *>(g + (size_t)r * cols + c) = *reinterpret_cast<const V *>(A + r * pitch + c);
-        });
+    using V = typename Pair<T>::type;
+    if (d.N1 & 1) {
+        RowCol q(d.G1);
+        for (int i = threadIdx.x; i < d.G2 * d.G1; i += blockDim.x, q.next()) g[i] = A[q.r * pitch + wcol(d, q.c)];
         return;
     }
-    RowCol q(cols);
-    for (int i = threadIdx.x; i < rows * cols; i += blockDim.x, q.next()) g[i] = A[q.r * pitch + q.c];
-}
-
-template <class T>
-__device__ __forceinline__ void load_plane(T *A, int pitch, int rows, int cols, const T *g)
-{
-    RowCol q(cols);
-    for (int i = threadIdx.x; i < rows * cols; i += blockDim.x, q.next()) A[q.r * pitch + q.c] = g[i];
+    for_row_pairs(d.G2, d.G1, pitch, d.G1,
+                  [&](int so, int go) { *reinterpret_cast<V *>(g + go) = *reinterpret_cast<const V *>(A + so); });
 }
 
 // Owner of work item `it` when the items are laid out in runs, one run per
@@ -282,6 +289,13 @@ __device__ __forceinline__ void cp_async_elem(T *dst, const T *src, bool valid)
     else
         asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(src), "r"(n) : "memory");
 }
+template <class T>
+__device__ __forceinline__ void cp_async_one(T *dst, const T *src)
+{
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    if constexpr (sizeof(T) == 4) asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(src) : "memory");
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src) : "memory");
+}
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
 // point-pair copy global -> shared (8 bytes FP32, 16 bytes FP64), both addresses on a pair
@@ -308,17 +322,36 @@ __device__ __forceinline__ void cp_async_pair_z(T *dst, const T *src, bool valid
         asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(n) : "memory");
 }
 
-// load_plane through cp.async (A in shared memory); the caller waits
+// real-space plane Z1 (I2 rows, IP1 apart) into A; the caller waits
 template <class T>
-__device__ __forceinline__ void load_plane_async(T *A, int pitch, int rows, int cols, const T *g)
+__device__ __forceinline__ void load_real_async(T *A, int pitch, const Dims &d, const T *g)
 {
-    if (pair_rows(cols, g)) {
-        for_row_pairs(rows, cols, [&](int r, int c) { cp_async_pair(A + r * pitch + c, g + (size_t)r * cols + c); });
+    for_row_pairs(d.I2, (d.I1 + 1) & ~1, pitch, d.IP1, [&](int so, int go) { cp_async_pair(A + so, g + go); });
+}
+
+// dense wavelet plane into the shared layout, its pad column (odd N1) zero;
+// the caller waits.  ASYNC: through cp.async (the buffer is shared memory)
+template <class T, bool ASYNC>
+__device__ __forceinline__ void load_wavelet(T *B, int pitch, const Dims &d, const T *g)
+{
+    if (!(d.N1 & 1)) {
+        for_row_pairs(d.G2, d.G1, pitch, d.G1, [&](int so, int go) {
+            using V = typename Pair<T>::type;
+            if (ASYNC) cp_async_pair(B + so, g + go);
+            else *reinterpret_cast<V *>(B + so) = *reinterpret_cast<const V *>(g + go);
+        });
         return;
     }
-    RowCol q(cols);
-    for (int i = threadIdx.x; i < rows * cols; i += blockDim.x, q.next())
-        cp_async_elem(A + q.r * pitch + q.c, g + i, true);
+    RowCol q(d.G1);
+    for (int i = threadIdx.x; i < d.G2 * d.G1; i += blockDim.x, q.next()) {
+        T *b = B + q.r * pitch + wcol(d, q.c);
+        if (ASYNC) cp_async_elem(b, g + i, true);
+        else *b = g[i];
+    }
+    for (int r = threadIdx.x; r < d.G2; r += blockDim.x) {
+        B[r * pitch + d.N1] = T(0);
+        B[r * pitch + d.H1 + d.N1] = T(0);
+    }
 }
 
 // gather_plane through cp.async (no scaling, same element type); the caller
@@ -326,27 +359,17 @@ __device__ __forceinline__ void load_plane_async(T *A, int pitch, int rows, int 
 template <class T, int S3>
 __device__ __forceinline__ void gather_plane_async_s(T *A, int pitch, const LrDev &L, int i3, const T *psi)
 {
-    const int H1 = half_off(L.N[0]), H2 = half_off(L.N[1]);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    if (!S3) {
-        const int a = L.plane_c[i3], b = L.plane_c[i3 + 1];
-        for (int sg = a + warp; sg < b; sg += nw) {
-            const int4 d = L.seg_c[sg];
-            for (int t = lane; t < d.z; t += 32) cp_async_elem(A + d.y * pitch + d.x + t, psi + d.w + t, true);
-        }
-    }
+    const PlaneCells p(L, pitch, i3, !S3);
+#pragma unroll 4
+    for (int j = p.a_c + threadIdx.x; j < p.b_c; j += blockDim.x) cp_async_one(A + L.pos_c[j], psi + j);
     const T *pf = psi + L.nvctr_c;
-    const int a = L.plane_f[i3], b = L.plane_f[i3 + 1];
-    for (int sg = a + warp; sg < b; sg += nw) {
-        const int4 d = L.seg_f[sg];
-        for (int t = lane; t < d.z; t += 32) {
-            const T *src = pf + 7 * (size_t)(d.w + t);
+#pragma unroll 4
+    for (int j = p.a_f + threadIdx.x; j < p.b_f; j += blockDim.x) {
+        T *a = A + L.pos_f[j];
+        const T *src = pf + 7 * (size_t)j;
 #pragma unroll
-            for (int c = 1; c <= 7; ++c) {
-                if (fs3(c) != S3) continue;
-                cp_async_elem(A + (fs2(c) * H2 + d.y) * pitch + fs1(c) * H1 + d.x + t, src + c - 1, true);
-            }
-        }
+        for (int c = 1; c <= 7; ++c)
+            if (fs3(c) == S3) cp_async_one(a + comp_ofs(c, p.H1, p.wrow), src + c - 1);
     }
 }
 
@@ -383,8 +406,8 @@ __host__ __device__ constexpr int plane_min_blocks(bool fp32, bool persist, int 
 // forms the search direction while it gathers it (dir 1: d = r, the first
 // iteration; dir 2: d = beta d + r with beta = rrn / rr, in T), and
 // writes d back; K3 accumulates <d | A d> of its plane, into one partial per
-// plane (as <P | W> of the fine planes it holds, since analysis is the
-// transpose of synthesis).  dir 0 / d null: plain gather / scatter.
+// plane (as <D | W> of the scaled plane D = D^-1/2 d that it holds and
+// W = (c + T) D).  dir 0 / d null: plain gather / scatter.
 template <class T> struct CgIo {
     T *d;
     const T *r;
@@ -392,51 +415,70 @@ template <class T> struct CgIo {
     int dir;
 };
 
-// The direction update on one gathered plane: A holds d (or zeros when
-// first), R the residual r of the same positions at row pitch rpitch = G1
-// (dense, so it fits in the transposed-plane buffer); every coefficient
-// position of the plane gets v = r (first) or beta d + r, written back to d
-// in global memory and into A scaled by D^-1/2.
+// The CG direction of wavelet plane kz, formed while it is gathered: every
+// coefficient gets v = r (first) or beta d + r, written back to d and into A
+// scaled by D^-1/2.  A thread loads the d and r values of two cells before it
+// stores any (a store to d would hold back the next cell's loads).
 template <class T, int S3>
-__device__ __forceinline__ void cg_dir_plane_s(T *A, int pitch, const T *R, int rpitch, const LrDev &L, int i3,
-                                               T *__restrict__ d, T beta, bool first, const T *sc)
+__device__ __forceinline__ void cg_dir_plane_s(T *A, int pitch, const LrDev &L, int i3, T *d, const T *__restrict__ r,
+                                               T beta, bool first, const T *sc)
 {
-    const int H1 = half_off(L.N[0]), H2 = half_off(L.N[1]);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    if (!S3) {
-        const int a = L.plane_c[i3], b = L.plane_c[i3 + 1];
-        for (int sg = a + warp; sg < b; sg += nw) {
-            const int4 q = L.seg_c[sg];
-            for (int t = lane; t < q.z; t += 32) {
-                const int pa = q.y * pitch + q.x + t, pr = q.y * rpitch + q.x + t;
-                const T v = first ? R[pr] : fma(beta, A[pa], R[pr]);
-                d[q.w + t] = v;
-                A[pa] = v * sc[0];
+    const PlaneCells p(L, pitch, i3, !S3);
+    constexpr int K = 2, NC = S3 ? 4 : 3, C0 = S3 ? 4 : 1;
+    const int nt = blockDim.x;
+    for (int j0 = p.a_c + threadIdx.x; j0 < p.b_c; j0 += 4 * nt) {
+        T v[4];
+        int at[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int j = j0 + k * nt;
+            if (j < p.b_c) {
+                at[k] = L.pos_c[j];
+                v[k] = first ? r[j] : fma(beta, d[j], r[j]);
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int j = j0 + k * nt;
+            if (j < p.b_c) {
+                d[j] = v[k];
+                A[at[k]] = v[k] * sc[0];
             }
         }
     }
     T *df = d + L.nvctr_c;
-    const int a = L.plane_f[i3], b = L.plane_f[i3 + 1];
-    for (int sg = a + warp; sg < b; sg += nw) {
-        const int4 q = L.seg_f[sg];
-        for (int t = lane; t < q.z; t += 32) {
-            T *dst = df + 7 * (size_t)(q.w + t);
+    const T *rf = r + L.nvctr_c;
+    for (int j0 = p.a_f + threadIdx.x; j0 < p.b_f; j0 += K * nt) {
+        T v[K][NC];
+        int at[K];
 #pragma unroll
-            for (int c = 1; c <= 7; ++c) {
-                if (fs3(c) != S3) continue;
-                const int pa = (fs2(c) * H2 + q.y) * pitch + fs1(c) * H1 + q.x + t;
-                const int pr = (fs2(c) * H2 + q.y) * rpitch + fs1(c) * H1 + q.x + t;
-                const T v = first ? R[pr] : fma(beta, A[pa], R[pr]);
-                dst[c - 1] = v;
-                A[pa] = v * sc[c];
+        for (int k = 0; k < K; ++k) {
+            const int j = j0 + k * nt;
+            if (j < p.b_f) {
+                at[k] = L.pos_f[j];
+                const size_t i = 7 * (size_t)j + C0 - 1;
+#pragma unroll
+                for (int c = 0; c < NC; ++c) v[k][c] = first ? rf[i + c] : fma(beta, df[i + c], rf[i + c]);
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            const int j = j0 + k * nt;
+            if (j < p.b_f) {
+                const size_t i = 7 * (size_t)j + C0 - 1;
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+                    df[i + c] = v[k][c];
+                    A[at[k] + comp_ofs(C0 + c, p.H1, p.wrow)] = v[k][c] * sc[C0 + c];
+                }
             }
         }
     }
 }
 
 // ---------------------------------------------------------------------------
-// K1: compressed psi -> P = S_x S_y psi (not in MODE_LOCDEN) and
-// Q = M_x M_y P (not in MODE_PRECOND) for one wavelet z-plane.
+// K1: compressed psi -> D, its wavelet plane (not in MODE_LOCDEN), and
+// Q = B_y B_x D (not in MODE_PRECOND) for one wavelet z-plane.
 //
 // Plane kernels (K1, K3) hold two plane buffers A and B in shared memory.
 // When two planes do not fit (FP64 boxes above about 60^3 periodic / 45^3
@@ -444,6 +486,10 @@ __device__ __forceinline__ void cg_dir_plane_s(T *A, int pitch, const T *R, int 
 // grid is one CTA per SM looping over the work items (PERSIST; the slice is
 // indexed by blockIdx, so no two running CTAs share it).  Otherwise every CTA
 // runs one item.
+//
+// The x pass walks rows (one thread per row and segment, scalar multiply-adds),
+// the y pass columns (two FP32 columns or one FP64 column a thread) and writes
+// its outputs straight to global memory: lanes hold neighbouring columns.
 template <class T, class TI, bool ALLPER, int MODE>
 __device__ __forceinline__ void k1_item(const LrDev *__restrict__ lrs, const OrbDev *__restrict__ orbs,
                                         const int *__restrict__ pre, int norb, const TI *__restrict__ psi,
@@ -451,7 +497,7 @@ __device__ __forceinline__ void k1_item(const LrDev *__restrict__ lrs, const Orb
                                         T *bslice, const CgIo<T> &cg)
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    constexpr int SEG = Seg<T>::v;
+    using U = typename ColUnit<T>::U;
     {
         const int oi = find_owner(pre, norb, it);   // item = (orbital, wavelet plane kz)
         const int kz = it - pre[oi];
@@ -466,20 +512,13 @@ __device__ __forceinline__ void k1_item(const LrDev *__restrict__ lrs, const Orb
         zero_region(A, d.G2, pitch);
         __syncthreads();
         if (MODE == MODE_PRECOND && cg.dir && std::is_same<T, TI>::value) {
-            // the CG direction, updated and scaled on the way in: d and r of
-            // the plane arrive by cp.async (d into A, r into B at pitch G1,
-            // which the transposed-plane buffer always holds)
+            // the CG direction, updated and scaled on the way in
             T *dv = cg.d + o.psi;
+            const T *rv = cg.r + o.psi;
             const bool first = cg.dir == 1;
             const T beta = first ? T(0) : (T)(cg.rrn[oi] / cg.rr[oi]);
-            if (!first) gather_plane_async<T>(A, pitch, L, kz, dv);
-            // (B in a global slice: plain loads, cp.async writes shared memory only)
-            if (bslice) gather_plane<T, T>(B, d.G1, L, kz, cg.r + o.psi, nullptr);
-            else gather_plane_async<T>(B, d.G1, L, kz, cg.r + o.psi);
-            cp_async_wait_all();
-            __syncthreads();
-            if (kz >= d.N3) cg_dir_plane_s<T, 1>(A, pitch, B, d.G1, L, kz - d.N3, dv, beta, first, sc);
-            else cg_dir_plane_s<T, 0>(A, pitch, B, d.G1, L, kz, dv, beta, first, sc);
+            if (kz >= d.N3) cg_dir_plane_s<T, 1>(A, pitch, L, kz - d.N3, dv, rv, beta, first, sc);
+            else cg_dir_plane_s<T, 0>(A, pitch, L, kz, dv, rv, beta, first, sc);
         } else if constexpr (std::is_same<T, TI>::value) {
             gather_plane_async<T>(A, pitch, L, kz, in_ptr(o, psi));
             cp_async_wait_all();
@@ -487,28 +526,30 @@ __device__ __forceinline__ void k1_item(const LrDev *__restrict__ lrs, const Orb
                 // D^-1/2 per component k = s1 + 2 s2 + 4 s3 of each plane position
                 __syncthreads();
                 const int s3 = kz >= d.N3 ? 4 : 0;
-                RowCol q(d.G1);
-                for (int i = threadIdx.x; i < d.G2 * d.G1; i += blockDim.x, q.next())
-                    A[q.r * pitch + q.c] *= sc[(q.c >= d.H1 ? 1 : 0) + (q.r >= d.H2 ? 2 : 0) + s3];
+                RowCol q(2 * d.H1);
+                for (int i = threadIdx.x; i < d.G2 * 2 * d.H1; i += blockDim.x, q.next())
+                    A[q.r * pitch + q.c] *= sc[(q.c >= d.H1 ? 1 : 0) + (q.r >= d.N2 ? 2 : 0) + s3];
             }
         } else {
             gather_plane<T, TI>(A, pitch, L, kz, in_ptr(o, psi), MODE == MODE_PRECOND ? sc : nullptr);
         }
         __syncthreads();
-        const int pt = d.pitchT(d.G2), ptf = d.pitchT(d.F2);
-        pass_syn<T, SEG, true>(A, B, xpose_geom(d.G2, pitch, pt), d.N1, d.H1, d.p1);   // S_x: G2 rows, G1 -> F1, into B^T
-        __syncthreads();
-        pass_syn<T, SEG, true>(B, A, xpose_geom(d.F1, pt, pitch), d.N2, d.H2, d.p2);   // S_y: F1 lines, G2 -> F2, into A
-        __syncthreads();
-        if (MODE != MODE_LOCDEN) store_plane(A, pitch, d.F2, d.F1, scratch + o.sP + (size_t)kz * d.F2 * d.F1);
+        if (MODE != MODE_LOCDEN) store_wavelet(A, pitch, d, scratch + o.sP + (size_t)kz * d.G2 * d.G1);
         if (MODE == MODE_PRECOND) return;
-        if (d.p1) pass_mf<T, SEG, 0, true>(A, B, xpose_geom(d.F2, pitch, ptf), d.F1, d.I1);   // M_x into B^T
-        else pass_mf<T, SEG, 2, true>(A, B, xpose_geom(d.F2, pitch, ptf), d.F1, d.I1);
+        row_b<T, kSeg>(A, B, d.G2, pitch, d.N1, d.H1, d.p1);   // B_x into B: G2 rows of I1 points
         __syncthreads();
-        if (d.p2) pass_mf<T, SEG, 0, true>(B, A, xpose_geom(d.I1, ptf, pitch), d.F2, d.I2);   // M_y into A
-        else pass_mf<T, SEG, 2, true>(B, A, xpose_geom(d.I1, ptf, pitch), d.F2, d.I2);
-        __syncthreads();
-        store_plane(A, pitch, d.I2, d.I1, scratch + o.sQ + (size_t)kz * d.I2 * d.I1);
+        // B_y: columns of B, G2 -> I2 points, to the Q plane
+        T *q = scratch + o.sQ + (size_t)kz * d.I2 * d.IP1;
+        const int npair = d.p2 ? d.N2 : d.N2 + 15;
+        for_items((d.I1 + U::n - 1) / U::n, (npair + kSeg - 1) / kSeg, [&](int u, int s) {
+            const int u0 = s * kSeg;
+            typename U::V acc[2 * kSeg];
+            col_b<U, kSeg>(acc, B + u * U::n, pitch, d.N2, d.N2, d.p2, u0);
+            T *o = q + (size_t)(2 * u0) * d.IP1 + u * U::n;
+#pragma unroll
+            for (int t = 0; t < 2 * kSeg; ++t)
+                if (2 * u0 + t < d.I2) *reinterpret_cast<typename U::V *>(o + t * d.IP1) = acc[t];
+        });
     }
 }
 
@@ -534,99 +575,59 @@ __global__ void __launch_bounds__(NT, plane_min_blocks(sizeof(T) == 4, PERSIST, 
 }
 
 // ---------------------------------------------------------------------------
-// Passes along the z-pencils of a TC-column tile (columns side by side, z
-// points TC apart): FP32 as line pairs with packed FMAs (wvlh_pairs.cuh),
-// FP64 one line per thread (FP64 has no packed FMA, and its pairs would
-// double the registers a thread holds).
-template <class T>
-__device__ __forceinline__ void z_syn(const T *src, T *dst, int N, int per)
-{
-    if constexpr (sizeof(T) == 4) pass2_syn<kPairSeg>(src, dst, PairGeom{TC / 2, TC, TC}, N, N, per);
-    else pass_syn<T, Seg<T>::v>(src, dst, LineGeom{TC, 1, TC, 1, TC}, N, N, per);
-}
-template <class T>
-__device__ __forceinline__ void z_ana(const T *src, T *dst, int N, int per)
-{
-    if constexpr (sizeof(T) == 4) pass2_ana<kPairSeg>(src, dst, PairGeom{TC / 2, TC, TC}, N, N, per);
-    else pass_ana<T, Seg<T>::v>(src, dst, LineGeom{TC, 1, TC, 1, TC}, N, N, per);
-}
-template <class T, int MODE>
-__device__ __forceinline__ void z_mf(const T *src, T *dst, int Lin, int Lout)
-{
-    if constexpr (sizeof(T) == 4) pass2_mf<kPairSeg, MODE>(src, dst, PairGeom{TC / 2, TC, TC}, Lin, Lout);
-    else pass_mf<T, Seg<T>::v, MODE>(src, dst, LineGeom{TC, 1, TC, 1, TC}, Lin, Lout);
-}
-template <class T, bool EN = true>
-__device__ __forceinline__ void z_kin(const T *src, T *dst, int L, int per, double scale, double *e)
-{
-    if constexpr (sizeof(T) == 4)
-        pass2_kin<kPairSeg, false, EN>(src, dst, PairGeom{TC / 2, TC, TC}, L, per, scale, 0.f, e);
-    else pass_kin<T, Seg<T>::v, false, false, EN>(src, dst, LineGeom{TC, 1, TC, 1, TC}, L, per, scale, T(0), e);
-}
-
-// ---------------------------------------------------------------------------
-// K2: z-pencil tiles, one kernel instance per chain (each half the code of a
-// two-chain kernel, which eases instruction fetch).  CHAIN 0:
-// Z1 = A_z Mt_z (V . M_z S_z Q) in place of Q, E_pot partial.  CHAIN 1:
-// Z2 = A_z K_z S_z P, E_kin(z) partial.
-// NT threads per CTA: 256, or for FP32 320 / 384, which give the passes over
-// 80- and 96-point z lines (32 line pairs x 10 or 12 eight-point segments)
-// one item per thread; resident CTAs per SM at 64 registers a thread.
-__host__ __device__ constexpr int z_min_blocks(bool fp32, int nt) { return fp32 ? 65536 / (64 * nt) : 1; }
+// K2: z-pencil tiles, one kernel instance per chain.  CHAIN 0:
+// Z1 = B^T_z (V . B_z Q) in place of Q, E_pot partial.  CHAIN 1: Z2 = T_z D,
+// E_kin(z) partial.  CHAIN 2: chain 1 without the energy (the preconditioner's
+// operator).
+// A tile is TC columns of the plane times the whole z extent, columns side by
+// side; a thread takes one column unit (two FP32 columns or one FP64 column)
+// of one z segment.  Chain 0 keeps the tile and its real-space form in shared
+// memory, chain 1 the tile alone; both write their outputs straight to global
+// memory, lanes on neighbouring columns.
+// NT threads per CTA: 256, or for FP32 320 / 384.
+__host__ __device__ constexpr int z_min_blocks(bool fp32, int nt) { return fp32 ? (nt > 256 ? 2 : 3) : 2; }
 
 template <class T, class TV, bool ALLPER, int CHAIN, int NT = kZThreads>
 __global__ void __launch_bounds__(NT, z_min_blocks(sizeof(T) == 4, NT)) k2_zpencil(const LrDev *__restrict__ lrs, const OrbDev *__restrict__ orbs,
                                                         const int *__restrict__ pre, int norb,
                                                         const TV *__restrict__ pot, T *__restrict__ scratch,
                                                         double *__restrict__ part_pot, double *__restrict__ part_kin,
-                                                        int part_stride, const __grid_constant__ CUtensorMap tm_in,
-                                                        const __grid_constant__ CUtensorMap tm_out, int tma)
+                                                        int part_stride, const __grid_constant__ CUtensorMap tm_in, int tma)
 {
-    // dynamic shared memory only (A, B, then the reduction slots and the TMA
-    // barrier), so that the tile buffer starts the block's shared window
+    // dynamic shared memory only (the tile, chain 0's real-space tile, then the
+    // reduction slots and the TMA barrier), so that the tile starts the
+    // block's shared window
     extern __shared__ __align__(128) unsigned char smem_raw[];
+    using U = typename ColUnit<T>::U;
+    using V = typename U::V;
     // item = (orbital, tile): chain 0 tiles the I1 x I2 plane of Q, chain 1
-    // the F1 x F2 plane of P, row-major; pre is the chain's own prefix table
-    // CHAIN 2: chain 1 without the energy (the preconditioner's operator)
+    // the G1 x G2 plane of D, row-major; pre is the chain's own prefix table
     constexpr int chain = CHAIN == 2 ? 1 : CHAIN;
     constexpr bool EN = CHAIN != 2;
+    constexpr int NU = TC / U::n, DS = NT / NU;   // column units, segments in flight
+    static_assert(NT % NU == 0, "whole segments per round");
     const int oi = find_owner(pre, norb, blockIdx.x);
     const int jj = blockIdx.x - pre[oi];   // tile index, also the energy slot
     const OrbDev o = orbs[oi];
     const LrDev L = lrs[o.lr];
     const Dims d(L, ALLPER);
-    const int ntx = chain == 0 ? (d.I1 + TX - 1) / TX : (d.F1 + TX - 1) / TX;
+    const int W = chain == 0 ? d.I1 : d.G1;   // plane width, height and row pitch of the data
+    const int H = chain == 0 ? d.I2 : d.G2;
+    const int WP = chain == 0 ? d.IP1 : d.G1;
+    const int ntx = (W + TX - 1) / TX;
     const int ty = jj / ntx, tx = jj - ty * ntx;
     const int x0 = tx * TX, y0 = ty * TY;
-    const int zl = max(d.G3, max(d.F3, d.I3));
     T *A = reinterpret_cast<T *>(smem_raw);
-    T *B = A + zl * TC;
-    double *red = reinterpret_cast<double *>(B + zl * TC);
+    T *B = A + d.G3 * TC;
+    double *red = reinterpret_cast<double *>(B + (chain == 0 ? d.I3 * TC : 0));
     uint64_t *tma_bar = reinterpret_cast<uint64_t *>(red + 32);
     // TMA writes the tile only into a kZAlign-aligned buffer
     tma = tma && !(smem_addr(A) & (kZAlign - 1));
-    const int W = chain == 0 ? d.I1 : d.F1;   // plane width/height of the data
-    const int H = chain == 0 ? d.I2 : d.F2;
-    T *g = scratch + (chain == 0 ? o.sQ : o.sP);
+    const T *g = scratch + (chain == 0 ? o.sQ : o.sP);
     T *gz = scratch + (chain == 0 ? o.sQ : o.sZ);
-    const size_t plane = (size_t)W * H;
-    // element loops: thread t owns tile column c = t % TC at z = t / TC + k ZS
-    constexpr int ZS = NT / TC;
-    const int col = threadIdx.x % TC, zs = threadIdx.x / TC;
-    const int xc = x0 + (col % TX), yc = y0 + (col / TX);
-    const bool inside = xc < W && yc < H;
-    const size_t colofs = (size_t)yc * W + xc;
+    const size_t plane = (size_t)WP * H;
 
-    // column pairs (x, x + 1) of one tile row move as point pairs when the
-    // plane rows have even length (the scratch planes start on a pair)
-    const bool pairs = pair_rows(W, g);
-    constexpr int TP = TC / 2, ZP = NT / TP;
-    const int pc = 2 * (threadIdx.x % TP), zp = threadIdx.x / TP;
-    const int xp = x0 + (pc % TX), yp = y0 + (pc / TX);
-    const bool pin = xp < W && yp < H;   // W even: x + 1 is inside too
-    const size_t pofs = (size_t)yp * W + xp;
-
-    // load the tile: TC columns x G3 z' rows, zero outside the plane
+    // load the tile: TC columns x G3 z rows, zero outside the plane
     if (tma) {
         // one box {32, 2, G3} of the batch's (x, y, z, orbital) scratch tensor
         if (threadIdx.x == 0) mbar_init(tma_bar, 1);
@@ -648,104 +649,103 @@ __global__ void __launch_bounds__(NT, z_min_blocks(sizeof(T) == 4, NT)) k2_zpenc
             return;
         }
     } else {
-        if (pairs) {
-            for (int z = zp; z < d.G3; z += ZP)
-                cp_async_pair_z(A + z * TC + pc, pin ? g + (size_t)z * plane + pofs : g, pin);
-        } else {
-            for (int z = zs; z < d.G3; z += ZS)
-                cp_async_elem(A + z * TC + col, inside ? g + (size_t)z * plane + colofs : g, inside);
-        }
+        // column pairs (x, x + 1) of one tile row: the rows have an even pitch
+        // and start on a pair
+        constexpr int TP = TC / 2, ZP = NT / TP;
+        const int pc = 2 * (threadIdx.x % TP);
+        const int xp = x0 + (pc % TX), yp = y0 + (pc / TX);
+        const bool pin = xp < W && yp < H;
+        const T *gp = pin ? g + (size_t)yp * WP + xp : g;
+        for (int z = threadIdx.x / TP; z < d.G3; z += ZP)
+            cp_async_pair_z(A + z * TC + pc, pin ? gp + (size_t)z * plane : g, pin);
         cp_async_wait_all();
         __syncthreads();
     }
+    // this thread's column unit; a pair may hang over the edge of a plane of
+    // odd width by the pad column (in1 false), never over the row's pitch
+    const int uc = (threadIdx.x % NU) * U::n, sg = threadIdx.x / NU;
+    const int xu = x0 + (uc % TX), yu = y0 + (uc / TX);
+    const bool in0 = xu < W && yu < H;
+    [[maybe_unused]] const bool in1 = in0 && xu + 1 < W;
+    gz += in0 ? (size_t)yu * WP + xu : 0;
     double e = 0.0;
-    z_syn<T>(A, B, d.N3, d.p3);                                   // S_z: G3 -> F3
-    __syncthreads();
     if constexpr (chain == 0) {
-        if (d.p3) z_mf<T, 0>(B, A, d.F3, d.I3);                   // M_z: F3 -> I3
-        else z_mf<T, 2>(B, A, d.F3, d.I3);
-        __syncthreads();
         // psir <- V psir, epot += V psir^2 (orbitals/potential.f90:1011-1031);
-        // per-thread partial sum in T, one FP64 conversion per thread (which
-        // z values a thread sums depends on the block size, so the energy's
-        // rounding does too)
-        const TV *V = o.pot_ptr ? (const TV *)o.pot_ptr : pot + o.pot;
+        // per-thread partial sum in T, one FP64 conversion per thread
+        const TV *pv = (o.pot_ptr ? (const TV *)o.pot_ptr : pot + o.pot);
+        const bool vpair = pair_rows(W, pv);
+        const size_t vplane = (size_t)W * H;
+        pv += in0 ? (size_t)yu * W + xu : 0;
         T ep = T(0);
-        constexpr int U = 4;   // potential loads in flight per thread
-        // thread t takes the column pair (x, x + 1) of pair index t % (TC/2) at
-        // z = t / (TC/2) + k ZP; the potential comes as a point pair when the
-        // rows are even and the buffer starts on a pair, else point by point.
-        // The arithmetic, and so the energy's summation order, is the same
-        // either way (it does not depend on where the potential lives).
-        using VV = typename Pair<TV>::type;
-        using P2 = typename Pair<T>::type;
-        const bool vpair = pairs && pair_rows(W, V);
-        const bool in0 = xp < W && yp < H, in1 = xp + 1 < W && yp < H;
-        const TV *vp = V + pofs;
-        for (int z0 = zp; z0 < d.I3; z0 += U * ZP) {
-            VV v[U];
+        const int npair = d.p3 ? d.N3 : d.N3 + 15;
+        for (int s = sg; s * kSeg < npair; s += DS) {
+            const int z0 = 2 * s * kSeg;
+            // the potential's points are on their way while the filter runs
+            V v[2 * kSeg], acc[2 * kSeg];
 #pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int z = z0 + u * ZP;
-                v[u].x = TV(0);
-                v[u].y = TV(0);
-                if (z < d.I3) {
-                    if (vpair) {
-                        if (in0) v[u] = *reinterpret_cast<const VV *>(vp + (size_t)z * plane);
+            for (int t = 0; t < 2 * kSeg; ++t) {
+                v[t] = U::zero();
+                if (z0 + t < d.I3 && in0) {
+                    const TV *a = pv + (size_t)(z0 + t) * vplane;
+                    if constexpr (U::n == 2) {
+                        if (vpair) {
+                            v[t] = *reinterpret_cast<const V *>(a);
+                        } else {
+                            v[t].x = a[0];
+                            if (in1) v[t].y = a[1];
+                        }
                     } else {
-                        if (in0) v[u].x = vp[(size_t)z * plane];
-                        if (in1) v[u].y = vp[(size_t)z * plane + 1];
+                        v[t] = a[0];
                     }
                 }
             }
+            col_b<U, kSeg>(acc, A + uc, TC, d.N3, d.N3, d.p3, s * kSeg);
+            V es = U::zero();
 #pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int z = z0 + u * ZP;
-                if (z < d.I3) {
-                    P2 *a = reinterpret_cast<P2 *>(A + z * TC + pc);
-                    P2 r = *a;
-                    const T w0 = (T)v[u].x * r.x, w1 = (T)v[u].y * r.y;
-                    if (in0) ep = fma(w0, r.x, ep);
-                    if (in1) ep = fma(w1, r.y, ep);
-                    r.x = in0 ? w0 : T(0);
-                    r.y = in1 ? w1 : T(0);
-                    *a = r;
+            for (int t = 0; t < 2 * kSeg; ++t) {
+                if (z0 + t < d.I3) {
+                    const V w = U::mulv(v[t], acc[t]);
+                    es = U::fmav(w, acc[t], es);
+                    *reinterpret_cast<V *>(B + (z0 + t) * TC + uc) = w;
                 }
             }
+            ep += U::sum(es);
         }
-        e += (double)ep;
+        e = (double)ep;
         __syncthreads();
-        if (d.p3) z_mf<T, 1>(A, B, d.I3, d.F3);                   // Mt_z: I3 -> F3
-        else z_mf<T, 3>(A, B, d.I3, d.F3);
-        __syncthreads();
-        z_ana<T>(B, A, d.N3, d.p3);                               // A_z: F3 -> G3
-    } else {
-        const double scale = -0.5 / ((0.5 * L.hgrid[2]) * (0.5 * L.hgrid[2]));
-        z_kin<T, EN>(B, A, d.F3, d.p3, scale, &e);                // K_z X
-        __syncthreads();
-        z_ana<T>(A, B, d.N3, d.p3);                               // A_z: F3 -> G3
-        __syncthreads();
-        T *t = A; A = B; B = t;                                   // result in A
-    }
-    if (tma) {
-        // the result tile goes back as one box (columns past the plane's
-        // edge are not written)
-        fence_async_smem();
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            tma_store_4d(&tm_out, x0, y0, 0, oi, A);
-            tma_store_drain();
+        for (int s = sg; s * kSeg < d.N3; s += DS) {
+            const int i0 = s * kSeg;
+            V c[kSeg], w[kSeg];
+            col_bt<U, kSeg>(c, w, B + uc, TC, d.I3, d.p3, i0);
+            if (in0) {
+#pragma unroll
+                for (int t = 0; t < kSeg; ++t)
+                    if (i0 + t < d.N3) {
+                        *reinterpret_cast<V *>(gz + (size_t)(i0 + t) * plane) = c[t];
+                        *reinterpret_cast<V *>(gz + (size_t)(d.N3 + i0 + t) * plane) = w[t];
+                    }
+            }
         }
     } else {
-        __syncthreads();
-        if (pairs) {
-            using V = typename Pair<T>::type;
-            if (pin)
-                for (int z = zp; z < d.G3; z += ZP)
-                    *reinterpret_cast<V *>(gz + (size_t)z * plane + pofs) =
-                        *reinterpret_cast<const V *>(A + z * TC + pc);
-        } else if (inside) {
-            for (int z = zs; z < d.G3; z += ZS) gz[(size_t)z * plane + colofs] = A[z * TC + col];
+        const double scale = -0.5 / (L.hgrid[2] * L.hgrid[2]);
+        for (int s = sg; s * kSeg < d.N3; s += DS) {
+            const int i0 = s * kSeg;
+            V c[kSeg], w[kSeg], es = U::zero();
+            Lags<U> lag;
+            col_t<U, kSeg, EN>(c, w, A + uc, TC, d.N3, d.N3, d.p3, i0, lag);
+            if (in0) {
+#pragma unroll
+                for (int t = 0; t < kSeg; ++t)
+                    if (i0 + t < d.N3) {
+                        if (EN) {
+                            es = U::fmav(c[t], *reinterpret_cast<const V *>(A + (i0 + t) * TC + uc), es);
+                            es = U::fmav(w[t], *reinterpret_cast<const V *>(A + (d.N3 + i0 + t) * TC + uc), es);
+                        }
+                        *reinterpret_cast<V *>(gz + (size_t)(i0 + t) * plane) = U::mul((T)scale, c[t]);
+                        *reinterpret_cast<V *>(gz + (size_t)(d.N3 + i0 + t) * plane) = U::mul((T)scale, w[t]);
+                    }
+                if (EN) e += ((double)U::sum(es) + (sizeof(T) == 4 ? lag.energy() : 0.0)) * scale;
+            }
         }
     }
     if constexpr (EN) {
@@ -756,8 +756,8 @@ __global__ void __launch_bounds__(NT, z_min_blocks(sizeof(T) == 4, NT)) k2_zpenc
 }
 
 // ---------------------------------------------------------------------------
-// K3 (MODE_LOCHAM): Hpsi plane kz = A_x A_y [Mt_x Mt_y Z1 + Z2 + (K_x + K_y) P]
-// K3 (MODE_PRECOND): D^-1/2 A_x A_y [Z2 + c P + (K_x + K_y) P]
+// K3 (MODE_LOCHAM): Hpsi plane kz = B^T_x B^T_y Z1 + (T_x + T_y) D + Z2
+// K3 (MODE_PRECOND): D^-1/2 [(c + T_x + T_y) D + Z2]
 template <class T, class TO, bool ALLPER, int MODE>
 __device__ __forceinline__ void k3_item(const LrDev *__restrict__ lrs, const OrbDev *__restrict__ orbs,
                                         const int *__restrict__ pre, int norb, const T *__restrict__ scratch,
@@ -766,7 +766,8 @@ __device__ __forceinline__ void k3_item(const LrDev *__restrict__ lrs, const Orb
                                         double *red, T *bslice, const TO *__restrict__ dotv)
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    constexpr int SEG = Seg<T>::v;
+    using U = typename ColUnit<T>::U;
+    using V = typename U::V;
     {
         const int oi = find_owner(pre, norb, it);   // item = (orbital, wavelet plane kz)
         const int kz = it - pre[oi];
@@ -776,81 +777,92 @@ __device__ __forceinline__ void k3_item(const LrDev *__restrict__ lrs, const Orb
         const int pitch = d.pitch();
         T *A = reinterpret_cast<T *>(smem_raw);
         T *B = bslice ? bslice : A + d.rows() * pitch;
+        const size_t wofs = (size_t)kz * d.G2 * d.G1;
 
         T cshift = T(0);
         if (MODE == MODE_PRECOND) {
             cshift = (T)cprec[oi];
             if (threadIdx.x < 8) sc[threadIdx.x] = (T)prec_scal(L, cprec[oi], threadIdx.x);
         } else {
-            load_plane_async(A, pitch, d.I2, d.I1, scratch + o.sQ + (size_t)kz * d.I2 * d.I1);
+            load_real_async(A, pitch, d, scratch + o.sQ + (size_t)kz * d.I2 * d.IP1);
             cp_async_wait_all();
             __syncthreads();
-            if (d.p1) pass_mf<T, SEG, 1, true>(A, B, xpose_geom(d.I2, pitch, d.pitchT(d.I2)), d.I1, d.F1);   // Mt_x into B^T
-            else pass_mf<T, SEG, 3, true>(A, B, xpose_geom(d.I2, pitch, d.pitchT(d.I2)), d.I1, d.F1);
+            // B^T_y: columns of A, I2 -> G2 points, into B
+            for_items((d.I1 + U::n - 1) / U::n, (d.N2 + kSeg - 1) / kSeg, [&](int u, int s) {
+                const int i0 = s * kSeg;
+                V c[kSeg], w[kSeg];
+                col_bt<U, kSeg>(c, w, A + u * U::n, pitch, d.I2, d.p2, i0);
+                T *b = B + i0 * pitch + u * U::n;
+#pragma unroll
+                for (int t = 0; t < kSeg; ++t)
+                    if (i0 + t < d.N2) {
+                        *reinterpret_cast<V *>(b + t * pitch) = c[t];
+                        *reinterpret_cast<V *>(b + (d.N2 + t) * pitch) = w[t];
+                    }
+            });
             __syncthreads();
-            // Mt_y into A, plus Z2 (read from global memory as the outputs are stored)
-            const T *z2 = scratch + o.sZ + (size_t)kz * d.F2 * d.F1;
-            if (d.p2) pass_mf<T, SEG, 1, true, true>(B, A, xpose_geom(d.F1, d.pitchT(d.I2), pitch), d.I2, d.F2, z2, d.F1);
-            else pass_mf<T, SEG, 3, true, true>(B, A, xpose_geom(d.F1, d.pitchT(d.I2), pitch), d.I2, d.F2, z2, d.F1);
+            row_bt<T, kSeg>(B, A, d.G2, pitch, d.I1, d.N1, d.H1, d.p1);   // B^T_x: I1 -> G1 points, into A
             __syncthreads();
         }
-        {
-            const T *z2 = scratch + o.sZ + (size_t)kz * d.F2 * d.F1;
-            const T *p = scratch + o.sP + (size_t)kz * d.F2 * d.F1;
-            const int nf = d.F2 * d.F1;
-            if (MODE != MODE_PRECOND && !bslice) {
-                // P -> B (Z2 is already in A)
-                load_plane_async(B, pitch, d.F2, d.F1, p);
-                cp_async_wait_all();
-            } else if (MODE == MODE_PRECOND && !bslice) {
-                // P -> B and Z2 -> A asynchronously (the x kinetic pass adds c P)
-                load_plane_async(B, pitch, d.F2, d.F1, p);
-                load_plane_async(A, pitch, d.F2, d.F1, z2);
-                cp_async_wait_all();
-            } else {
-                RowCol q(d.F1);
-                for (int i = threadIdx.x; i < nf; i += blockDim.x, q.next()) {
-                    const int e = q.r * pitch + q.c;
-                    const T pv = p[i];
-                    if (MODE == MODE_PRECOND) A[e] = z2[i];   // (MODE_LOCHAM: Z2 came with Mt_y)
-                    B[e] = pv;
-                }
-            }
-        }
+        if (bslice) load_wavelet<T, false>(B, pitch, d, scratch + o.sP + wofs);
+        else load_wavelet<T, true>(B, pitch, d, scratch + o.sP + wofs);
+        cp_async_wait_all();
         __syncthreads();
-        // e: the kinetic energy partial (MODE_LOCHAM) or <d | A d> (MODE_PRECOND)
-        // (the preconditioner's operator has no energy: its kinetic passes
-        // are compiled without the energy terms, and its x pass adds c P)
+        // e: the kinetic energy partial (MODE_LOCHAM) or <d | A d>
+        // (MODE_PRECOND), which with D = D^-1/2 d is <D, W> for the plane
+        // W = (c + T) D before its scaling
         constexpr bool EN = MODE != MODE_PRECOND;
         double e = 0.0;
-        const double sx = -0.5 / ((0.5 * L.hgrid[0]) * (0.5 * L.hgrid[0]));
-        const double sy = -0.5 / ((0.5 * L.hgrid[1]) * (0.5 * L.hgrid[1]));
-        pass_kin<T, SEG, true, true, EN, !EN>(B, A, rows_geom(d.F2, pitch), d.F1, d.p1, sx, cshift, &e);   // += K_x P
+        const double sx = -0.5 / (L.hgrid[0] * L.hgrid[0]);
+        const double sy = -0.5 / (L.hgrid[1] * L.hgrid[1]);
+        row_t<T, kSeg, EN, EN>(B, A, d.G2, pitch, d.N1, d.H1, d.p1, sx, cshift, &e);
         __syncthreads();
-        // += K_y P: the lines along y are the plane's columns, side by side
-        // (F1 is even): FP32 takes them in pairs with packed FMAs
-        if constexpr (sizeof(T) == 4) pass2_kin<kPairSeg, true, EN>(B, A, PairGeom{d.F1 / 2, pitch, pitch}, d.F2, d.p2, sy, 0.f, &e);
-        else pass_kin<T, SEG, true, false, EN>(B, A, cols_geom(d.F1, pitch), d.F2, d.p2, sy, T(0), &e);
-        __syncthreads();
-        if (MODE == MODE_PRECOND && dotv) {
-            // <d | A d> of this plane without reading d: analysis is the
-            // transpose of synthesis, so <d, D^-1/2 A_x A_y W> = <P, W> with
-            // P = S_x S_y D^-1/2 d (in B) and W the fine plane now in A
-            RowCol q(d.F1);
-            for (int i = threadIdx.x; i < d.F2 * d.F1; i += blockDim.x, q.next()) {
-                const int el = q.r * pitch + q.c;
-                e = fma((double)B[el], (double)A[el], e);
-            }
-            __syncthreads();   // A_x overwrites B
-        }
-        pass_ana<T, SEG, true>(A, B, xpose_geom(d.F2, pitch, d.pitchT(d.F2)), d.N1, d.H1, d.p1);   // A_x: F1 -> G1, into B^T
-        __syncthreads();
-        pass_ana<T, SEG, true>(B, A, xpose_geom(d.G1, d.pitchT(d.F2), pitch), d.N2, d.H2, d.p2);   // A_y: F2 -> G2, into A
+        // + T_y D + Z2, the plane's columns
+        const T *z2 = scratch + o.sZ + wofs;
+        const bool odd = d.N1 & 1;
+        for_items(2 * d.H1 / U::n, (d.N2 + kSeg - 1) / kSeg, [&](int u, int sg) {
+            const int i0 = sg * kSeg, col = u * U::n;
+            // this unit's columns in the dense Z2 plane (none for a pad column)
+            const int g0 = col < d.H1 ? col : col - d.H1 + d.N1;
+            const bool h0 = col != d.N1 && col != d.H1 + d.N1;
+            const int g1 = col + 1 < d.H1 ? col + 1 : col + 1 - d.H1 + d.N1;
+            const bool h1 = col + 1 != d.N1 && col + 1 != d.H1 + d.N1;
+            V s[kSeg], w[kSeg], es = U::zero();
+            Lags<U> lag;
+            col_t<U, kSeg, EN>(s, w, B + col, pitch, d.N2, d.N2, d.p2, i0, lag);
+            auto put = [&](int row, V conv) {
+                const T *zr = z2 + (size_t)row * d.G1;
+                V z;
+                if constexpr (U::n == 2) {
+                    if (!odd) {
+                        z = *reinterpret_cast<const V *>(zr + g0);
+                    } else {
+                        z.x = h0 ? zr[g0] : T(0);
+                        z.y = h1 ? zr[g1] : T(0);
+                    }
+                } else {
+                    z = !odd || h0 ? zr[g0] : T(0);
+                }
+                V *a = reinterpret_cast<V *>(A + row * pitch + col);
+                const V x = *reinterpret_cast<const V *>(B + row * pitch + col);
+                const V r = U::fma((T)sy, conv, U::add(*a, z));
+                *a = r;
+                if (EN) es = U::fmav(x, conv, es);
+                else if (dotv) U::dot(e, x, r, odd ? h0 : true, odd ? h1 : true);
+            };
+#pragma unroll
+            for (int t = 0; t < kSeg; ++t)
+                if (i0 + t < d.N2) {
+                    put(i0 + t, s[t]);
+                    put(d.N2 + i0 + t, w[t]);
+                }
+            if (EN) e += ((double)U::sum(es) + (sizeof(T) == 4 ? lag.energy() : 0.0)) * sy;
+        });
         __syncthreads();
         scatter_plane<T, TO>(A, pitch, L, kz, out_ptr(o, hpsi), accumulate != 0, MODE == MODE_PRECOND ? sc : nullptr);
         const double s = block_sum(e, red);
         // slots 0 .. ntx1*nty1-1 belong to the z kernel's chain-1 tiles
-        const int slot = ((d.F1 + TX - 1) / TX) * ((d.F2 + TY - 1) / TY) + kz;
+        const int slot = ((d.G1 + TX - 1) / TX) * ((d.G2 + TY - 1) / TY) + kz;
         if (threadIdx.x == 0 && part_kin) part_kin[(size_t)oi * part_stride + slot] = s;
     }
 }
@@ -927,17 +939,20 @@ __global__ void __launch_bounds__(kZThreads) kd_density(const LrDev *__restrict_
     const Dims d(L, ALLPER);
     const int ntx = (d.I1 + TX - 1) / TX;
     const int x0 = (j % ntx) * TX, y0 = (j / ntx) * TY;
-    const int zl = max(d.G3, max(d.F3, d.I3));
     T *A = reinterpret_cast<T *>(smem_raw);
-    T *B = A + zl * TC;
+    T *B = A + d.G3 * TC;
     const int W = d.I1, H = d.I2;
-    const size_t plane = (size_t)W * H;
-    // thread t owns tile column c = t % TC at z = t / TC + k ZS
-    constexpr int ZS = kZThreads / TC;
-    const int col = threadIdx.x % TC, zs = threadIdx.x / TC;
-    const int xc = x0 + (col % TX), yc = y0 + (col / TX);
-    const bool inside = xc < W && yc < H;
-    const size_t colofs = (size_t)yc * W + xc;
+    using U = typename ColUnit<T>::U;
+    constexpr int NU = TC / U::n, DS = kZThreads / NU;
+    const size_t plane = (size_t)d.IP1 * H;
+    // column pairs as point pairs (even row pitch)
+    constexpr int TP = TC / 2, ZP = kZThreads / TP;
+    const int pc = 2 * (threadIdx.x % TP);
+    const int xp = x0 + (pc % TX), yp = y0 + (pc / TX);
+    const bool pin = xp < W && yp < H;
+    const size_t pofs = pin ? (size_t)yp * d.IP1 + xp : 0;
+    const int uc = (threadIdx.x % NU) * U::n;
+    const int npair = d.p3 ? d.N3 : d.N3 + 15;
     double acc[MAXP];
 #pragma unroll
     for (int k = 0; k < MAXP; ++k) acc[k] = 0.0;
@@ -946,32 +961,24 @@ __global__ void __launch_bounds__(kZThreads) kd_density(const LrDev *__restrict_
         const OrbDev o = orbs[orb];
         const T *g = scratch + o.sQ;
         __syncthreads();
-        if (pair_rows(W, g)) {
-            // column pairs as point pairs (even plane rows)
-            constexpr int TP = TC / 2, ZP = kZThreads / TP;
-            const int pc = 2 * (threadIdx.x % TP), zp = threadIdx.x / TP;
-            const int xp = x0 + (pc % TX), yp = y0 + (pc / TX);
-            const bool pin = xp < W && yp < H;
-            const size_t pofs = (size_t)yp * W + xp;
-            for (int z = zp; z < d.G3; z += ZP)
-                cp_async_pair_z(A + z * TC + pc, pin ? g + (size_t)z * plane + pofs : g, pin);
-        } else {
-            for (int z = zs; z < d.G3; z += ZS)
-                cp_async_elem(A + z * TC + col, inside ? g + (size_t)z * plane + colofs : g, inside);
-        }
+        for (int z = threadIdx.x / TP; z < d.G3; z += ZP)
+            cp_async_pair_z(A + z * TC + pc, g + (pin ? (size_t)z * plane + pofs : 0), pin);
         cp_async_wait_all();
         __syncthreads();
-        z_syn<T>(A, B, d.N3, d.p3);                               // S_z
-        __syncthreads();
-        if (d.p3) z_mf<T, 0>(B, A, d.F3, d.I3);                   // M_z
-        else z_mf<T, 2>(B, A, d.F3, d.I3);
+        for (int s = threadIdx.x / NU; s * kSeg < npair; s += DS) {
+            typename U::V r[2 * kSeg];
+            col_b<U, kSeg>(r, A + uc, TC, d.N3, d.N3, d.p3, s * kSeg);
+#pragma unroll
+            for (int t = 0; t < 2 * kSeg; ++t)
+                if (2 * s * kSeg + t < d.I3) *reinterpret_cast<typename U::V *>(B + (2 * s * kSeg + t) * TC + uc) = r[t];
+        }
         __syncthreads();
         const double hf = hfac[orb];
 #pragma unroll
         for (int k = 0; k < MAXP; ++k) {
             const int i = threadIdx.x + k * blockDim.x;
             if (i < d.I3 * TC) {
-                const double r = (double)A[i];
+                const double r = (double)B[i];
                 acc[k] = fma(hf * r, r, acc[k]);
             }
         }
@@ -1217,12 +1224,12 @@ static auto k3_for(const PlaneCfg &pc) -> decltype(&k3_plane_backward<T, TO, ALL
 
 // TMA maps of the z kernel's tiles: when every orbital of the batch lies in
 // one region, the scratch planes of all orbitals form regular 4-D tensors
-// (x, y, z, orbital) for Q (chain 0, read and written in place), P (chain 1
-// input) and Z2 (chain 1 output); otherwise (several regions, or rows whose
-// byte length TMA cannot stride) the tiles move with cp.async.
+// (x, y, z, orbital) for Q (chain 0) and D (chain 1); otherwise (several
+// regions, or rows whose byte length TMA cannot stride) the tiles move with
+// cp.async.
 struct ZMaps {
-    CUtensorMap q, p, z;
-    int ok = 0;
+    CUtensorMap q, p;
+    int okq = 0, okp = 0;
 };
 template <class T>
 static void zmaps(const Plan &p, T *scratch, ZMaps &m)
@@ -1230,12 +1237,9 @@ static void zmaps(const Plan &p, T *scratch, ZMaps &m)
     memset(&m, 0, sizeof(m));
     if (p.orb_scratch <= 0) return;
     const int es = (int)sizeof(T);
-    const long long G3 = p.tile_dims[0], F1 = p.tile_dims[1], F2 = p.tile_dims[2], I1 = p.tile_dims[3],
-                    I2 = p.tile_dims[4];
-    const long long sQ0 = G3 * F2 * F1, sZ0 = sQ0 + G3 * I2 * I1;
-    m.ok = encode_tile_map(&m.q, scratch + sQ0, es, I1, I2, G3, p.norb, p.orb_scratch) &&
-           encode_tile_map(&m.p, scratch, es, F1, F2, G3, p.norb, p.orb_scratch) &&
-           encode_tile_map(&m.z, scratch + sZ0, es, F1, F2, G3, p.norb, p.orb_scratch);
+    const TileDims &t = p.tile;
+    m.okq = encode_tile_map(&m.q, scratch + t.ofs_q, es, t.I1, t.IP1, t.I2, t.G3, p.norb, p.orb_scratch);
+    m.okp = encode_tile_map(&m.p, scratch, es, t.G1, t.G1, t.G2, t.G3, p.norb, p.orb_scratch);
 }
 
 // K1 / K3 launch with the plane configuration of the batch
@@ -1267,8 +1271,8 @@ static cudaError_t run_k3(const Plan &p, const PlaneCfg &pc, const T *scratch, T
 // K2 launch with the block size zt (FP32: 256, 320 or 384; FP64: 256)
 template <class T, class TV, bool ALLPER, int CHAIN>
 static cudaError_t run_k2(int zt, int nwork, size_t sm2, const Plan &p, const int *pre, const TV *pot, T *scratch,
-                          double *part_pot, double *part_kin, int part_stride, const CUtensorMap &m_in,
-                          const CUtensorMap &m_out, int tma, cudaStream_t st)
+                          double *part_pot, double *part_kin, int part_stride, const CUtensorMap &m_in, int tma,
+                          cudaStream_t st)
 {
     auto k = k2_zpencil<T, TV, ALLPER, CHAIN, kZThreads>;
     if constexpr (sizeof(T) == 4) {
@@ -1281,7 +1285,7 @@ static cudaError_t run_k2(int zt, int nwork, size_t sm2, const Plan &p, const in
     cudaError_t err;
     if ((err = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm2))) return err;
     k<<<nwork, zt, sm2, st>>>(p.d_lr, p.d_orb, pre, p.norb, pot, scratch, part_pot, part_kin, part_stride, m_in,
-                              m_out, tma);
+                              tma);
     return cudaSuccess;
 }
 
@@ -1302,7 +1306,7 @@ static cudaError_t launch_locham_bc(const Plan &p, const TIO *psi, const TIO *po
 {
     const int fp = sizeof(T) == 8 ? 1 : 0;
     const PlaneCfg pc = plane_cfg(p, fp, p.n_work13);
-    const size_t sm2 = p.smem2[fp] + kZExtra;
+    const size_t sm2 = p.smem_z0[fp] + kZExtra, sm2p = p.smem_z1[fp] + kZExtra;
     T *gtmp = pc.global_b ? scratch + p.scratch_elems : nullptr;
     cudaError_t err;
     cudaMemsetAsync(part_pot, 0, sizeof(double) * (size_t)p.norb * p.part_stride, st);
@@ -1314,9 +1318,9 @@ static cudaError_t launch_locham_bc(const Plan &p, const TIO *psi, const TIO *po
     if ((err = run_k1<T, TIO, ALLPER, MODE_LOCHAM>(p, pc, psi, scratch, nullptr, gtmp, st))) return err;
     if (ev) cudaEventRecord(ev[1], st);
     if ((err = run_k2<T, TIO, ALLPER, 0>(p.z_threads[fp], p.n_work2, sm2, p, p.d_pre2, pot, scratch, part_pot,
-                                         part_kin, p.part_stride, zm.q, zm.q, zm.ok, st)) ||
-        (err = run_k2<T, TIO, ALLPER, 1>(p.z_threads[fp], p.n_work2p, sm2, p, p.d_pre2p, pot, scratch, part_pot,
-                                         part_kin, p.part_stride, zm.p, zm.z, zm.ok, st)))
+                                         part_kin, p.part_stride, zm.q, zm.okq, st)) ||
+        (err = run_k2<T, TIO, ALLPER, 1>(p.z_threads[fp], p.n_work2p, sm2p, p, p.d_pre2p, pot, scratch, part_pot,
+                                         part_kin, p.part_stride, zm.p, zm.okp, st)))
         return err;
     if (ev) cudaEventRecord(ev[2], st);
     if ((err = run_k3<T, TIO, ALLPER, MODE_LOCHAM>(p, pc, scratch, hpsi, part_kin, p.part_stride, accumulate, nullptr,
@@ -1340,12 +1344,12 @@ cudaError_t launch_locham(const Plan &p, const TIO *psi, const TIO *pot, TIO *hp
                                            st, ev);
 }
 
-#ifdef WVLH_FUSED_F32
+#if defined(WVLH_FUSED_F32) && defined(WVLH_FUSED_LOCHAM)
 template cudaError_t launch_locham<float, float>(const Plan &, const float *, const float *, float *, float *,
                                                  double *, double *, double *, double *, int, cudaStream_t,
                                                  cudaEvent_t *);
 #endif
-#ifdef WVLH_FUSED_F64
+#if defined(WVLH_FUSED_F64) && defined(WVLH_FUSED_LOCHAM)
 template cudaError_t launch_locham<double, double>(const Plan &, const double *, const double *, double *, double *,
                                                    double *, double *, double *, double *, int, cudaStream_t,
                                                    cudaEvent_t *);
@@ -1357,7 +1361,7 @@ static cudaError_t launch_locden_bc(const Plan &p, const T *psi, const double *h
 {
     const int fp = sizeof(T) == 8 ? 1 : 0;
     const PlaneCfg pc = plane_cfg(p, fp, p.n_work13);
-    const size_t sm2 = p.smem2[fp] + kZExtra;
+    const size_t sm2 = p.smem_z0[fp] + kZExtra;
     T *gtmp = pc.global_b ? scratch + p.scratch_elems : nullptr;
     cudaError_t err;
     auto kd = p.den_acc > 32 ? kd_density<T, ALLPER, 48> : kd_density<T, ALLPER, 32>;
@@ -1378,11 +1382,11 @@ cudaError_t launch_locden(const Plan &p, const T *psi, const double *hfac, doubl
     if (p.all_periodic) return launch_locden_bc<T, true>(p, psi, hfac, rho, scratch, part, st);
     return launch_locden_bc<T, false>(p, psi, hfac, rho, scratch, part, st);
 }
-#ifdef WVLH_FUSED_F32
+#if defined(WVLH_FUSED_F32) && defined(WVLH_FUSED_LOCDEN)
 template cudaError_t launch_locden<float>(const Plan &, const float *, const double *, double *, float *, double *,
                                           cudaStream_t);
 #endif
-#ifdef WVLH_FUSED_F64
+#if defined(WVLH_FUSED_F64) && defined(WVLH_FUSED_LOCDEN)
 template cudaError_t launch_locden<double>(const Plan &, const double *, const double *, double *, double *,
                                            double *, cudaStream_t);
 #endif
@@ -1397,14 +1401,14 @@ static cudaError_t launch_prec_apply_bc(const Plan &p, const T *x, T *y, const d
     const int fp = sizeof(T) == 8 ? 1 : 0;
     PlaneCfg pc = plane_cfg(p, fp, p.n_work13);
     if (!pc.global_b) pc.threads = p.plane_threads_pre[fp];
-    const size_t sm2 = p.smem2[fp] + kZExtra;
+    const size_t sm2 = p.smem_z1[fp] + kZExtra;
     T *gtmp = pc.global_b ? scratch + p.scratch_elems : nullptr;
     cudaError_t err;
     if ((err = run_k1<T, T, ALLPER, MODE_PRECOND>(p, pc, x, scratch, cprec, gtmp, st, cg))) return err;
     ZMaps zm;
     zmaps(p, scratch, zm);
     if ((err = run_k2<T, T, ALLPER, 2>(p.z_threads_pre[fp], p.n_work2p, sm2, p, p.d_pre2p, (const T *)nullptr, scratch,
-                                       nullptr, nullptr, 0, zm.p, zm.z, zm.ok, st)))
+                                       nullptr, nullptr, 0, zm.p, zm.okp, st)))
         return err;
     if (dotpart) cudaMemsetAsync(dotpart, 0, sizeof(double) * (size_t)p.norb * p.part_stride, st);
     if ((err = run_k3<T, T, ALLPER, MODE_PRECOND>(p, pc, scratch, y, dotpart, dotpart ? p.part_stride : 0, 0, cprec,
@@ -1475,11 +1479,11 @@ cudaError_t launch_precond(const Plan &p, int ncong, const double *cprec, T *x, 
     return vec ? cg_loop<T, true>(p, ncong, cprec, x, b, r, dvec, ad, rr, dad, rrn, part, dotpart, hist, apply, st)
                : cg_loop<T, false>(p, ncong, cprec, x, b, r, dvec, ad, rr, dad, rrn, part, dotpart, hist, apply, st);
 }
-#ifdef WVLH_FUSED_F32
+#if defined(WVLH_FUSED_F32) && defined(WVLH_FUSED_PRECOND)
 template cudaError_t launch_precond<float>(const Plan &, int, const double *, float *, const float *, float *, float *,
                                            float *, float *, double *, double *, cudaStream_t);
 #endif
-#ifdef WVLH_FUSED_F64
+#if defined(WVLH_FUSED_F64) && defined(WVLH_FUSED_PRECOND)
 template cudaError_t launch_precond<double>(const Plan &, int, const double *, double *, const double *, double *,
                                             double *, double *, double *, double *, double *, cudaStream_t);
 #endif

@@ -24,10 +24,12 @@ __host__ __device__ constexpr int plane_ctas_per_sm(bool fp32, int nt)
                 : (nt >= 384 ? 1 : nt >= 256 ? 2 : 4);
 }
 
-// CTA size of the plane kernels, chosen per batch by a small occupancy model:
-// a pass has `rows` lines of up to `len` points cut into segments of SEG
-// outputs; with nt threads it takes ceil(items / nt) rounds, so the busy
-// fraction is items / (rounds nt); the SM holds as many CTAs as registers (the
+// CTA size of the plane kernels, chosen per batch by a small occupancy model.
+// A pass over rows has `rows` lines, one over columns len lines (two FP32
+// columns or one FP64 column a thread), each cut into segments of 12 points;
+// with nt threads a pass of n items takes ceil(n / nt) rounds, so the busy
+// fraction is the two passes' items over their rounds times nt (a column item
+// of two FP32 columns weighs two); the SM holds as many CTAs as registers (the
 // compiled count above), shared memory and threads allow.  The expected rate
 // is busy x resident threads x ctas / (ctas + 1/2) — the last factor because
 // a CTA's barrier waits are covered only by the other resident CTAs; each
@@ -42,16 +44,17 @@ inline int choose_plane_threads(const std::vector<PlaneShape> &shapes, bool fp32
     const int cand64[4] = {512, kPlaneThreads, 256, 128};
     const int *cand = fp32 ? cand32 : cand64;
     const int ncand = fp32 ? 5 : 4;
-    const int seg = fp32 ? 8 : 4;
+    const long long seg = 12, cu = fp32 ? 2 : 1;
     double best = 0.0;
     int pick = 0;
     for (int k = 0; k < ncand; ++k) {
         const int nt = cand[k];
         double cost = 0.0;
         for (const PlaneShape &s : shapes) {
-            const long long items = s.rows * ((s.len + seg - 1) / seg);
-            const long long rounds = (items + nt - 1) / nt;
-            const double busy = (double)items / (double)(rounds * nt);
+            const long long ri = s.rows * ((s.len + seg - 1) / seg);
+            const long long ci = (s.len + cu - 1) / cu * ((s.rows + seg - 1) / seg);
+            const long long rounds = (ri + nt - 1) / nt + cu * ((ci + nt - 1) / nt);
+            const double busy = (double)(ri + cu * ci) / (double)(rounds * nt);
             const long long by_regs = plane_ctas_per_sm(fp32, nt);
             const long long by_smem = (227LL * 1024) / (s.smem_bytes + 1024);
             const long long by_threads = 2048 / nt;
@@ -71,17 +74,19 @@ inline int choose_plane_threads(const std::vector<PlaneShape> &shapes, bool fp32
 constexpr int kZThreads = 256;
 
 // One localisation region (box + compressed-key tables) as seen by kernels.
-// Segments are decoded once on upload from the reference's 1-based keyg/keyv
-// (wavelib/un-compress.f90:896-905 arithmetic) into {i0, i2, len, jj0}, with
-// jj0 the 0-based compressed position; plane_c/plane_f[i3..i3+1] delimit the
-// segments of coarse z-plane i3 (keys are sorted by linear index).
+// The reference's 1-based keyg/keyv (wavelib/un-compress.f90:896-905) are
+// expanded on upload to one word per cell: pos_c / pos_f[j] is the place of the
+// j-th coarse / fine cell of the compressed vector in a wavelet plane of the
+// plane kernels' shared-memory layout (y * pitch + x).  Keys are sorted, so the
+// cells of one z-plane are consecutive: plane_c / plane_f[i3 .. i3+1] delimit
+// those of coarse plane i3.
 struct LrDev {
     int N[3];
     int per[3];
     int nseg_c, nseg_f;
     int nvctr_c, nvctr_f;
-    const int4 *seg_c;
-    const int4 *seg_f;
+    const int *pos_c;
+    const int *pos_f;
     const int *plane_c;  // N3+1 entries
     const int *plane_f;  // N3+1 entries
     double hgrid[3];     // coarse grid spacing
@@ -93,15 +98,22 @@ struct OrbDev {
     int pad;
     long long psi;   // element offset of [psi_c | psi_f] in the psi/hpsi arrays
     long long pot;   // element offset of this orbital's potential / density (ISF grid)
-    long long sP;    // scratch element offsets: P (G3*F2*F1)
-    long long sQ;    //   Q / Z1 (G3*I2*I1)
-    long long sZ;    //   Z2 (G3*F2*F1)
+    // scratch element offsets of the orbital's planes, one per wavelet z-plane:
+    long long sP;    //   D (2N2 x 2N1 dense)
+    long long sQ;    //   Q / Z1 (I2 rows, isf_pitch apart)
+    long long sZ;    //   Z2 (2N2 x 2N1 dense)
     double c;        // shift of (T + c), preconditioner only
     // optional absolute buffers (a batch that spans several owners' arrays);
     // when set they replace base + offset
     const void *in_ptr;
     void *out_ptr;
     const void *pot_ptr;
+};
+
+// plane shapes of a batch whose orbitals all lie in one region (TMA tiles)
+struct TileDims {
+    long long G1, G2, G3, I1, IP1, I2;
+    long long ofs_q;   // Q's element offset in an orbital's scratch
 };
 
 enum FusedMode { MODE_LOCHAM = 0, MODE_LOCDEN = 1, MODE_PRECOND = 2 };
@@ -155,11 +167,12 @@ struct Plan {
     int z_threads_pre[2] = {kZThreads, kZThreads};   // the same for the preconditioner operator
     size_t smem2[2] = {0, 0};
     int pitch_max = 0, rows_max = 0, zlen_max = 0;
+    size_t smem_z0[2] = {0, 0};    // dynamic smem bytes of the z kernel's chain 0 (and the density) ...
+    size_t smem_z1[2] = {0, 0};    // ... and of chain 1
     // scratch elements per orbital when every orbital lies in one region (the
-    // planes then form regular (x, y, z, orbital) tensors: TMA tiles), else 0;
-    // tile_dims = {G3, F1, F2, I1, I2} of that region
+    // planes then form regular (x, y, z, orbital) tensors: TMA tiles), else 0
     long long orb_scratch = 0;
-    long long tile_dims[5] = {0, 0, 0, 0, 0};
+    TileDims tile = {};
     std::vector<void *> owned;     // device allocations to free
 };
 

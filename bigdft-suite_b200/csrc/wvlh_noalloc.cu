@@ -32,29 +32,23 @@ using namespace wvlh;
 // address on the current device is obtained with cudaGetSymbolAddress.
 constexpr size_t kNoAllocBytes = size_t(64) << 20;
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocBytes];
+// Cell tables of the coarse and the fine keys beside it.  A box that fits the
+// scratch has at least 96 bytes of it per coarse cell (three FP32 planes of
+// eight points), which bounds the cells of either key set.
+constexpr size_t kNoAllocCells = kNoAllocBytes / 96 + 1;
+static __device__ int g_noalloc_cells[2 * kNoAllocCells];
 
 namespace {
 
 constexpr int kMaxDevices = 64;
 std::mutex g_setup_mutex;
 void *g_scratch_addr[kMaxDevices] = {nullptr};
+void *g_cells_addr[kMaxDevices] = {nullptr};
 
-// decoded segment {i0, i2, len, jj0} from 1-based keys (un-compress.f90:896-905)
-__global__ void k_decode_segments(int n1, int n2, int nseg, const int32_t *__restrict__ keyg,
-                                  const int32_t *__restrict__ keyv, int4 *__restrict__ seg)
-{
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= nseg) return;
-    const int j0 = keyg[2 * s], j1 = keyg[2 * s + 1];
-    int ii = j0 - 1;
-    const int i3 = ii / (n1 * n2);
-    ii -= i3 * n1 * n2;
-    const int i2 = ii / n1;
-    seg[s] = make_int4(ii - i2 * n1, i2, j1 - j0 + 1, keyv[s] - 1);
-}
-
-// first segment of each coarse z-plane (keys are sorted by linear index)
-__global__ void k_plane_ranges(int n12, int n3, int nseg, const int32_t *__restrict__ keyg, int *__restrict__ plane)
+// compressed index of the first cell at or after each coarse z-plane (keys are
+// sorted by linear index)
+__global__ void k_plane_ranges(int n12, int n3, int nseg, int nvctr, const int32_t *__restrict__ keyg,
+                               const int32_t *__restrict__ keyv, int *__restrict__ plane)
 {
     const int i3 = blockIdx.x * blockDim.x + threadIdx.x;
     if (i3 > n3) return;
@@ -63,7 +57,7 @@ __global__ void k_plane_ranges(int n12, int n3, int nseg, const int32_t *__restr
         const int mid = (lo + hi) >> 1;
         if ((keyg[2 * mid] - 1) / n12 < i3) lo = mid + 1; else hi = mid;
     }
-    plane[i3] = lo;
+    plane[i3] = lo < nseg ? keyv[lo] - 1 : nvctr;
 }
 
 // work tables of one orbital: {0, G3} plane-kernel items, {0, n2} and {0, n2p}
@@ -121,17 +115,19 @@ extern "C" int wvlh_locham_noalloc(int precision, const int n[3], const int peri
     }
     const size_t es = precision == 32 ? 4 : 8;
     const int ntx0 = (I[0] + TX_ - 1) / TX_, nty0 = (I[1] + TY_ - 1) / TY_;
-    const int ntx1 = (F[0] + TX_ - 1) / TX_, nty1 = (F[1] + TY_ - 1) / TY_;
+    const int ntx1 = (G[0] + TX_ - 1) / TX_, nty1 = (G[1] + TY_ - 1) / TY_;
     const int stride = (ntx0 * nty0 > ntx1 * nty1 + G[2]) ? ntx0 * nty0 : ntx1 * nty1 + G[2];
-    const long long sP = (long long)G[2] * F[1] * F[0], sQ = (long long)G[2] * I[1] * I[0];
+    const OrbScratch sc = orb_scratch(N, per);
     // layout of the static array
     size_t off = 0;
     const size_t o_lr = off; off = up256(off + sizeof(LrDev));
     const size_t o_orb = off; off = up256(off + sizeof(OrbDev));
     const size_t o_kc = off; off = up256(off + 8 * (size_t)nseg_c + 4 * (size_t)nseg_c);
     const size_t o_kf = off; off = up256(off + 8 * (size_t)nseg_f + 4 * (size_t)nseg_f);
-    const size_t o_sc = off; off = up256(off + 16 * (size_t)nseg_c);
-    const size_t o_sf = off; off = up256(off + 16 * (size_t)nseg_f);
+    // room of 16 bytes a segment: not used by the tables below, it counts
+    // towards which boxes the entry point takes
+    off = up256(off + 16 * (size_t)nseg_c);
+    off = up256(off + 16 * (size_t)nseg_f);
     const size_t o_pc = off; off = up256(off + 4 * (size_t)(N[2] + 1));
     const size_t o_pf = off; off = up256(off + 4 * (size_t)(N[2] + 1));
     const size_t o_w13 = off; off = up256(off + 2 * sizeof(int));
@@ -139,19 +135,20 @@ extern "C" int wvlh_locham_noalloc(int precision, const int n[3], const int peri
     const size_t o_w2p = off; off = up256(off + 2 * sizeof(int));
     const size_t o_pp = off; off = up256(off + 8 * (size_t)stride);
     const size_t o_pk = off; off = up256(off + 8 * (size_t)stride);
-    const size_t o_scr = off; off = up256(off + es * (size_t)(2 * sP + sQ));
+    const size_t o_scr = off; off = up256(off + es * (size_t)sc.total);
     if (off > kNoAllocBytes) {
         set_last_error(WVLH_ERR_TOO_LARGE);
         return WVLH_ERR_TOO_LARGE;
     }
     // plane buffers as the fused kernels lay them out (coarse_width, vec_pitch)
     const int W1 = coarse_width(N[0]), W2 = coarse_width(N[1]);
-    const size_t width = (size_t)(W1 > F[0] ? (W1 > I[0] ? W1 : I[0]) : (F[0] > I[0] ? F[0] : I[0]));
-    const size_t pitch = (size_t)vec_pitch((int)width);
+    const size_t pitch = (size_t)plane_pitch(N[0], per[0]);
     const size_t rows = (size_t)(W2 > F[1] ? (W2 > I[1] ? W2 : I[1]) : (F[1] > I[1] ? F[1] : I[1]));
     const size_t zl = (size_t)(G[2] > F[2] ? (G[2] > I[2] ? G[2] : I[2]) : (F[2] > I[2] ? F[2] : I[2]));
-    // second plane buffer: P (F2 rows x pitch) or a transposed plane, each
-    // pass's lines along x at the vec_pitch of its y length
+    // second plane buffer: 2 N2 rows (usedB); the room of the largest plane or
+    // transposed plane on the fine and real-space grids (planeB) decides which
+    // boxes the entry point takes
+    const size_t usedB = (size_t)G[1] * pitch;
     size_t planeB = (size_t)F[1] * pitch;
     const size_t uses[4] = {(size_t)F[0] * vec_pitch(W2), (size_t)I[0] * vec_pitch(F[1]),
                             (size_t)F[0] * vec_pitch(I[1]), (size_t)W1 * vec_pitch(F[1])};
@@ -173,6 +170,7 @@ extern "C" int wvlh_locham_noalloc(int precision, const int n[3], const int peri
     // kept for the life of the process (the library does not support a reset
     // of the device, which would reload its module, while it is loaded)
     unsigned char *base;
+    int *cells;
     {
         std::lock_guard<std::mutex> lock(g_setup_mutex);
         if (!g_scratch_addr[dev]) {
@@ -181,8 +179,15 @@ extern "C" int wvlh_locham_noalloc(int precision, const int n[3], const int peri
                 set_last_error(WVLH_ERR_CUDA);
                 return WVLH_ERR_CUDA;
             }
+            void *t = nullptr;
+            if (cudaGetSymbolAddress(&t, g_noalloc_cells) != cudaSuccess || !t) {
+                set_last_error(WVLH_ERR_CUDA);
+                return WVLH_ERR_CUDA;
+            }
+            g_cells_addr[dev] = t;
             g_scratch_addr[dev] = a;
         }
+        cells = (int *)g_cells_addr[dev];
         base = (unsigned char *)g_scratch_addr[dev];
     }
     cudaStream_t st = (cudaStream_t)stream;
@@ -196,8 +201,8 @@ extern "C" int wvlh_locham_noalloc(int precision, const int n[3], const int peri
     L.nseg_f = nseg_f;
     L.nvctr_c = (int)nvc;
     L.nvctr_f = (int)nvf;
-    L.seg_c = (const int4 *)(base + o_sc);
-    L.seg_f = (const int4 *)(base + o_sf);
+    L.pos_c = cells;
+    L.pos_f = cells + kNoAllocCells;
     L.plane_c = (const int *)(base + o_pc);
     L.plane_f = (const int *)(base + o_pf);
     OrbDev O;
@@ -206,8 +211,8 @@ extern "C" int wvlh_locham_noalloc(int precision, const int n[3], const int peri
     O.psi = 0;
     O.pot = 0;
     O.sP = 0;
-    O.sQ = sP;
-    O.sZ = sP + sQ;
+    O.sQ = sc.q;
+    O.sZ = sc.z;
     O.c = 0.0;
     O.in_ptr = nullptr;
     O.out_ptr = nullptr;
@@ -226,17 +231,19 @@ extern "C" int wvlh_locham_noalloc(int precision, const int n[3], const int peri
     if (nseg_c) {
         NA_CK(cudaMemcpyAsync(dkc, keyg_c, 8 * (size_t)nseg_c, cudaMemcpyHostToDevice, st));
         NA_CK(cudaMemcpyAsync(dkc + 2 * nseg_c, keyv_c, 4 * (size_t)nseg_c, cudaMemcpyHostToDevice, st));
-        k_decode_segments<<<(nseg_c + 255) / 256, 256, 0, st>>>(N[0], N[1], nseg_c, dkc, dkc + 2 * nseg_c,
-                                                                (int4 *)(base + o_sc));
+        k_cell_places<<<(nseg_c + 7) / 8, 256, 0, st>>>(N[0], N[1], (int)pitch, nseg_c, dkc, dkc + 2 * nseg_c,
+                                                         cells);
     }
     if (nseg_f) {
         NA_CK(cudaMemcpyAsync(dkf, keyg_f, 8 * (size_t)nseg_f, cudaMemcpyHostToDevice, st));
         NA_CK(cudaMemcpyAsync(dkf + 2 * nseg_f, keyv_f, 4 * (size_t)nseg_f, cudaMemcpyHostToDevice, st));
-        k_decode_segments<<<(nseg_f + 255) / 256, 256, 0, st>>>(N[0], N[1], nseg_f, dkf, dkf + 2 * nseg_f,
-                                                                (int4 *)(base + o_sf));
+        k_cell_places<<<(nseg_f + 7) / 8, 256, 0, st>>>(N[0], N[1], (int)pitch, nseg_f, dkf, dkf + 2 * nseg_f,
+                                                         cells + kNoAllocCells);
     }
-    k_plane_ranges<<<(N[2] + 256) / 256, 256, 0, st>>>(N[0] * N[1], N[2], nseg_c, dkc, (int *)(base + o_pc));
-    k_plane_ranges<<<(N[2] + 256) / 256, 256, 0, st>>>(N[0] * N[1], N[2], nseg_f, dkf, (int *)(base + o_pf));
+    k_plane_ranges<<<(N[2] + 256) / 256, 256, 0, st>>>(N[0] * N[1], N[2], nseg_c, (int)nvc, dkc, dkc + 2 * nseg_c,
+                                                      (int *)(base + o_pc));
+    k_plane_ranges<<<(N[2] + 256) / 256, 256, 0, st>>>(N[0] * N[1], N[2], nseg_f, (int)nvf, dkf, dkf + 2 * nseg_f,
+                                                      (int *)(base + o_pf));
     k_work_lists<<<1, 32, 0, st>>>(G[2], ntx0 * nty0, ntx1 * nty1, (int *)(base + o_w13), (int *)(base + o_w2),
                                    (int *)(base + o_w2p));
     NA_CK(cudaGetLastError());
@@ -256,17 +263,21 @@ extern "C" int wvlh_locham_noalloc(int precision, const int n[3], const int peri
     p.part_stride = stride;
     p.plane_elems = (long long)(rows * pitch);
     {
-        const long long len = (long long)width, ab = (long long)(rows * pitch + planeB);
+        const long long len = (long long)pitch, ab = (long long)(rows * pitch + usedB);
         p.plane_threads[0] = choose_plane_threads({PlaneShape{(long long)rows, len, ab * 4, 1}}, true);
         p.plane_threads[1] = choose_plane_threads({PlaneShape{(long long)rows, len, ab * 8, 1}}, false);
     }
-    p.planeB_elems = (long long)planeB;
-    p.scratch_elems = 2 * sP + sQ;
-    p.smem13[0] = (rows * pitch + planeB) * 4;
-    p.smem13[1] = (rows * pitch + planeB) * 8;
+    p.planeB_elems = (long long)usedB;
+    p.scratch_elems = sc.total;
+    p.smem13[0] = (rows * pitch + usedB) * 4;
+    p.smem13[1] = (rows * pitch + usedB) * 8;
     p.smem2[0] = 2 * zl * TX_ * TY_ * 4;
     p.smem2[1] = 2 * zl * TX_ * TY_ * 8;
-    // the energy partials are cleared by the launcher; P, Q/Z1, Z2 are fully
+    for (int f = 0; f < 2; ++f) {
+        p.smem_z0[f] = (size_t)(G[2] + I[2]) * TX_ * TY_ * (f ? 8 : 4);
+        p.smem_z1[f] = (size_t)G[2] * TX_ * TY_ * (f ? 8 : 4);
+    }
+    // the energy partials are cleared by the launcher; D, Q/Z1, Z2 are fully
     // overwritten before they are read, so stale contents of an earlier call
     // never leak into this one
     if (precision == 64)

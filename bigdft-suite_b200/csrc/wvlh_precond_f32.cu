@@ -1,0 +1,4 @@
+// FP32 kernels and launcher of the preconditioner (wvlh_fused_impl.cuh).
+#define WVLH_FUSED_F32
+#define WVLH_FUSED_PRECOND
+#include "wvlh_fused_impl.cuh"

@@ -5,9 +5,9 @@
 // which is exactly the dense layout of a TMA box {32, 2, Z, 1} over the
 // 4-D tensor (x, y, z, orbital) of a batch's scratch planes.  One thread
 // issues the box load (cp.async.bulk.tensor, completion counted in bytes on
-// an mbarrier) and, at the end, the box store of the result; elements past
-// the plane's edge are zero-filled on load and skipped on store.  No
-// multicast is used (the source is this GPU's own memory).
+// an mbarrier); elements past the plane's edge are zero-filled.  The results
+// leave by ordinary stores, as the threads form them.  No multicast is used
+// (the source is this GPU's own memory).
 //
 // Every wait on the mbarrier is bounded: after kTmaSpinLimit polls the CTA
 // records an error in the batch's flag and returns without using the tile.
@@ -60,26 +60,10 @@ __device__ __forceinline__ void tma_load_4d(void *dst, const CUtensorMap *map, i
         : "memory");
 }
 
-// box store from shared memory; the caller fences the generic-proxy writes
-// (fence_async_smem) and a barrier precedes the call
-__device__ __forceinline__ void tma_store_4d(const CUtensorMap *map, int c0, int c1, int c2, int c3, const void *src)
-{
-    asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%1, %2, %3, %4}], [%5];\n" ::"l"(
-                     reinterpret_cast<uint64_t>(map)),
-                 "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(smem_addr(src))
-                 : "memory");
-    asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
-}
-
-// the issuing thread waits until the stores have read shared memory
-__device__ __forceinline__ void tma_store_drain() { asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory"); }
-
-// shared-memory writes by ordinary stores become visible to the TMA unit
-__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory"); }
-
-// Host: encode a 4-D map (x, y, z, orbital) over a batch's scratch planes,
-// box {32, 2, Z, 1}; false when the shapes or alignments do not allow TMA.
-bool encode_tile_map(CUtensorMap *map, const void *base, int elem_bytes, long long W, long long H, long long Z,
-                     long long norb, long long orb_stride_elems);
+// Host: encode a 4-D map (x, y, z, orbital) over a batch's scratch planes with
+// rows `pitch` elements apart, box {32, 2, Z, 1}; false when the shapes or
+// alignments do not allow TMA.
+bool encode_tile_map(CUtensorMap *map, const void *base, int elem_bytes, long long W, long long pitch, long long H,
+                     long long Z, long long norb, long long orb_stride_elems);
 
 }  // namespace wvlh
