@@ -241,9 +241,11 @@ static int region_make(int device, const wvlh_locreg &L, wvlh_region **out)
     pk.add(kvc, &r->keyv_c);
     pk.add(kgf, &r->keyg_f);
     pk.add(kvf, &r->keyv_f);
-    // the cell tables follow the uploaded block and are expanded on the device
+    // the cell tables follow the uploaded block and are expanded on the device;
+    // a box whose cells are all fine has one table for both key sets
+    const bool same = L.nseg_c == L.nseg_f && kgc == kgf;
     const size_t tab = (pk.img.size() + 255) & ~size_t(255);
-    if (cudaMalloc(&r->mem, tab + sizeof(int) * ((size_t)nvc + nvf)) != cudaSuccess) {
+    if (cudaMalloc(&r->mem, tab + sizeof(int) * ((size_t)nvc + (same ? 0 : nvf))) != cudaSuccess) {
         r->mem = nullptr;
         region_free(r);
         return WVLH_ERR_NOMEM;
@@ -255,12 +257,12 @@ static int region_make(int device, const wvlh_locreg &L, wvlh_region **out)
     pk.place(r->mem);
     int *pos = reinterpret_cast<int *>(static_cast<unsigned char *>(r->mem) + tab);
     d.pos_c = pos;
-    d.pos_f = pos + nvc;
+    d.pos_f = same ? pos : pos + nvc;
     const int pitch = plane_pitch(d.N[0], d.per[0]);
     if (L.nseg_c)
         k_cell_places<<<(L.nseg_c + 7) / 8, 256>>>(d.N[0], d.N[1], pitch, L.nseg_c, (const int32_t *)r->keyg_c,
                                                    (const int32_t *)r->keyv_c, pos);
-    if (L.nseg_f)
+    if (L.nseg_f && !same)
         k_cell_places<<<(L.nseg_f + 7) / 8, 256>>>(d.N[0], d.N[1], pitch, L.nseg_f, (const int32_t *)r->keyg_f,
                                                    (const int32_t *)r->keyv_f, pos + nvc);
     // launches may follow on any stream
@@ -387,6 +389,8 @@ static void layout(wvlh_batch *b, const std::vector<int> &orb_lr, const std::vec
         sm2_elems = std::max(sm2_elems, (size_t)2 * zl * TX_ * TY_);
         z0_elems = std::max(z0_elems, (size_t)(G3 + I3) * TX_ * TY_);
         z1_elems = std::max(z1_elems, (size_t)G3 * TX_ * TY_);
+        p.z_segs0 = std::max(p.z_segs0, ((d.per[2] ? N3 : N3 + 15) + kSegZ - 1) / kSegZ);
+        p.z_segs1 = std::max(p.z_segs1, (N3 + kSegZ - 1) / kSegZ);
     }
     p.psi_total = psi_off;
     p.all_periodic = true;
@@ -405,8 +409,8 @@ static void layout(wvlh_batch *b, const std::vector<int> &orb_lr, const std::vec
         }
     }
     p.part_stride = stride;
-    p.plane_threads[0] = choose_plane_threads(shapes32, true);
-    p.plane_threads[1] = choose_plane_threads(shapes64, false);
+    p.plane_threads[0] = choose_plane_threads(shapes32, true, p.plane_cand[0]);
+    p.plane_threads[1] = choose_plane_threads(shapes64, false, p.plane_cand[1]);
     p.plane_threads_pre[0] = p.plane_threads[0];
     p.plane_threads_pre[1] = p.plane_threads[1];
     apply_tuned(p);   // a measured choice for this shape, when wvlh_batch_autotune made one
@@ -828,9 +832,6 @@ static std::string tune_key(const Plan &p, int fp, bool pre = false, int what = 
     return k;
 }
 
-// the block sizes the plane kernels are compiled for
-static const int kTune32[5] = {1024, 512, kPlaneThreads, 256, 128};
-static const int kTune64[4] = {512, kPlaneThreads, 256, 128};
 // the block sizes the FP32 z kernel is compiled for
 static const int kTuneZ32[3] = {kZThreads, 320, 384};
 
@@ -897,8 +898,8 @@ extern "C" int wvlh_batch_autotune(wvlh_batch *b, int precision, const void *psi
     CK(cudaSetDevice(c->device));
     const int fp = precision == 64;
     auto call = [&] { return wvlh_locham_batched(b, precision, psi, pot, hpsi, ekin, epot, 0); };
-    int rc = time_candidates(c, &b->plan.plane_threads[fp], fp ? kTune64 : kTune32, fp ? 4 : 5, reps, call, chosen,
-                             cand, ms, ncand);
+    int rc = time_candidates(c, &b->plan.plane_threads[fp], b->plan.plane_cand[fp], 5, reps, call, chosen, cand, ms,
+                             ncand);
     // then the z kernel's block size (FP32), with the plane kernels' pick
     if (!rc && !fp) rc = time_candidates(c, &b->plan.z_threads[0], kTuneZ32, 3, reps, call, nullptr, nullptr, nullptr, nullptr);
     if (rc) return fail(rc);
@@ -926,8 +927,8 @@ extern "C" int wvlh_batch_autotune_precond(wvlh_batch *b, int precision, int nco
     CK(cudaSetDevice(c->device));
     const int fp = precision == 64;
     auto call = [&] { return wvlh_precond_batched(b, precision, ncong, cprec, x, rhs, nullptr); };
-    int rc = time_candidates(c, &b->plan.plane_threads_pre[fp], fp ? kTune64 : kTune32, fp ? 4 : 5, reps, call,
-                             chosen, cand, ms, ncand);
+    int rc = time_candidates(c, &b->plan.plane_threads_pre[fp], b->plan.plane_cand[fp], 5, reps, call, chosen, cand, ms,
+                             ncand);
     if (!rc && !fp)
         rc = time_candidates(c, &b->plan.z_threads_pre[0], kTuneZ32, 3, reps, call, nullptr, nullptr, nullptr, nullptr);
     if (rc) return fail(rc);

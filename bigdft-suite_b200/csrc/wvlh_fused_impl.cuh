@@ -52,11 +52,6 @@ constexpr int TC = TX * TY;
 constexpr int kZAlign = 128;
 constexpr int kZExtra = 32 * 8 + 16;
 
-// coarse points of one thread's segment, all passes and both precisions: six
-// give the 48-point lines of a 96 x 96 plane two full rounds of 384 threads
-// (rows) and one (columns), and a 32-column tile one round of 256
-constexpr int kSeg = 6;
-
 // A wavelet line holds N scaling and N wavelet coefficients.  In global memory
 // a wavelet plane is dense, G2 = 2 N2 rows of G1 = 2 N1 points.  In shared
 // memory the wavelet half of a row starts at the even offset H1 (rows move as
@@ -104,15 +99,51 @@ __device__ __forceinline__ double prec_scal(const LrDev &L, double c, int k)
 
 // The cells of a wavelet z-plane are consecutive in the compressed vector, and
 // each has its place in the shared plane in the region's cell table, so
-// gathering and scattering walk cells with all lanes busy, no segment in
-// sight.  (A warp per segment left a third of the lanes of 48-cell rows idle
-// and cost the plane kernels 45 to 50 instructions a point, more than one of
-// their filter passes.)  A fine cell holds the seven components c = s1 + 2 s2 +
-// 4 s3; a plane takes those of its own s3: the three after the coarse
-// coefficient (s3 = 0) or four (s3 = 1).
+// gathering and scattering walk the plane's values with all lanes busy, no
+// segment in sight.  (A warp per segment left a third of the lanes of 48-cell
+// rows idle and cost the plane kernels 45 to 50 instructions a point.)  A fine
+// cell holds the seven components c = s1 + 2 s2 + 4 s3; a plane takes those of
+// its own s3: the three after the coarse coefficient (s3 = 0) or the last four
+// (s3 = 1).  Where values are written, consecutive lanes take the components of
+// one cell, then the next cell's, so that a warp's store covers 11 or 8
+// neighbouring cells.  (One cell a lane put every store on 28 sectors, each
+// moved for four bytes: 36 of the 172 us of the preconditioner's K3 on
+// 24 x 48^3.)
 
 // value c (its s1, s2 bits) of a cell sits this far from the cell's place
 __device__ __forceinline__ int comp_ofs(int c, int H1, int wrow) { return fs1(c) * H1 + fs2(c) * wrow; }
+
+// f(j, place of cell j) for j = j0, j0 + step, ... < end, the places of K cells
+// read together: their latency would stand before every copy or store
+template <int K, class F>
+__device__ __forceinline__ void for_cells(int j0, int end, int step, const int *__restrict__ pos, F &&f)
+{
+    for (; j0 < end; j0 += K * step) {
+        int at[K];
+#pragma unroll
+        for (int k = 0; k < K; ++k)
+            if (j0 + k * step < end) at[k] = __ldg(pos + j0 + k * step);
+#pragma unroll
+        for (int k = 0; k < K; ++k)
+            if (j0 + k * step < end) f(j0 + k * step, at[k]);
+    }
+}
+
+// A thread's share of the fine values of a plane of s3 = S3: component c of the
+// cells j0, j0 + step, ... (up to two threads of a block stay out when a cell
+// gives three values)
+template <int S3> struct FineShare {
+    static constexpr int NC = S3 ? 4 : 3, C0 = S3 ? 4 : 1;
+    int j0, c, step;
+    bool in;
+    __device__ __forceinline__ FineShare()
+    {
+        step = blockDim.x / NC;
+        j0 = threadIdx.x / NC;
+        c = C0 + threadIdx.x - j0 * NC;
+        in = j0 < step;
+    }
+};
 
 struct PlaneCells {
     int a_c, b_c, a_f, b_f;   // the plane's coarse cells (none when s3 = 1), fine cells
@@ -136,15 +167,12 @@ __device__ __forceinline__ void gather_plane_s(T *A, int pitch, const LrDev &L, 
 {
     const PlaneCells p(L, pitch, i3, !S3);
     const T s0 = sc ? sc[0] : T(1);
-    for (int j = p.a_c + threadIdx.x; j < p.b_c; j += blockDim.x) A[L.pos_c[j]] = (T)psi[j] * s0;
-    const TI *pf = psi + L.nvctr_c;
-    for (int j = p.a_f + threadIdx.x; j < p.b_f; j += blockDim.x) {
-        T *a = A + L.pos_f[j];
-        const TI *src = pf + 7 * (size_t)j;
-#pragma unroll
-        for (int c = 1; c <= 7; ++c)
-            if (fs3(c) == S3) a[comp_ofs(c, p.H1, p.wrow)] = (T)src[c - 1] * (sc ? sc[c] : T(1));
-    }
+    for_cells<8>(p.a_c + threadIdx.x, p.b_c, blockDim.x, L.pos_c, [&](int j, int at) { A[at] = (T)psi[j] * s0; });
+    const FineShare<S3> w;
+    const TI *pf = psi + L.nvctr_c - 1 + w.c;
+    T *a = A + comp_ofs(w.c, p.H1, p.wrow);
+    const T sf = sc ? sc[w.c] : T(1);
+    for_cells<8>(p.a_f + w.j0, w.in ? p.b_f : 0, w.step, L.pos_f, [&](int j, int at) { a[at] = (T)pf[7 * (size_t)j] * sf; });
 }
 
 // the z component s3 of a plane is uniform over the CTA: one copy of the
@@ -163,23 +191,13 @@ __device__ __forceinline__ void scatter_plane_s(const T *A, int pitch, const LrD
 {
     const PlaneCells p(L, pitch, i3, !S3);
     const T s0 = sc ? sc[0] : T(1);
-#pragma unroll 2
-    for (int j = p.a_c + threadIdx.x; j < p.b_c; j += blockDim.x) {
-        const TO v = (TO)(A[L.pos_c[j]] * s0);
-        out[j] = accumulate ? out[j] + v : v;
-    }
-    TO *pf = out + L.nvctr_c;
-#pragma unroll 2
-    for (int j = p.a_f + threadIdx.x; j < p.b_f; j += blockDim.x) {
-        const T *a = A + L.pos_f[j];
-        TO *dst = pf + 7 * (size_t)j;
-#pragma unroll
-        for (int c = 1; c <= 7; ++c) {
-            if (fs3(c) != S3) continue;
-            const TO v = (TO)(a[comp_ofs(c, p.H1, p.wrow)] * (sc ? sc[c] : T(1)));
-            dst[c - 1] = accumulate ? dst[c - 1] + v : v;
-        }
-    }
+    auto put = [&](TO *dst, T v) { *dst = accumulate ? *dst + (TO)v : (TO)v; };
+    for_cells<8>(p.a_c + threadIdx.x, p.b_c, blockDim.x, L.pos_c, [&](int j, int at) { put(out + j, A[at] * s0); });
+    const FineShare<S3> w;
+    TO *pf = out + L.nvctr_c - 1 + w.c;
+    const T *a = A + comp_ofs(w.c, p.H1, p.wrow);
+    const T sf = sc ? sc[w.c] : T(1);
+    for_cells<8>(p.a_f + w.j0, w.in ? p.b_f : 0, w.step, L.pos_f, [&](int j, int at) { put(pf + 7 * (size_t)j, a[at] * sf); });
 }
 
 template <class T, class TO>
@@ -252,6 +270,26 @@ __device__ __forceinline__ void store_wavelet(const T *A, int pitch, const Dims 
     }
     for_row_pairs(d.G2, d.G1, pitch, d.G1,
                   [&](int so, int go) { *reinterpret_cast<V *>(g + go) = *reinterpret_cast<const V *>(A + so); });
+}
+
+// A += the dense wavelet plane g
+template <class T>
+__device__ __forceinline__ void add_wavelet(T *A, int pitch, const Dims &d, const T *__restrict__ g)
+{
+    if (d.N1 & 1) {
+        RowCol q(d.G1);
+        for (int i = threadIdx.x; i < d.G2 * d.G1; i += blockDim.x, q.next()) A[q.r * pitch + wcol(d, q.c)] += g[i];
+        return;
+    }
+    using V = typename Pair<T>::type;
+    for_row_pairs(d.G2, d.G1, pitch, d.G1, [&](int so, int go) {
+        const V v = *reinterpret_cast<const V *>(g + go);
+        V *a = reinterpret_cast<V *>(A + so);
+        V r = *a;
+        r.x += v.x;
+        r.y += v.y;
+        *a = r;
+    });
 }
 
 // Owner of work item `it` when the items are laid out in runs, one run per
@@ -360,17 +398,16 @@ template <class T, int S3>
 __device__ __forceinline__ void gather_plane_async_s(T *A, int pitch, const LrDev &L, int i3, const T *psi)
 {
     const PlaneCells p(L, pitch, i3, !S3);
-#pragma unroll 4
-    for (int j = p.a_c + threadIdx.x; j < p.b_c; j += blockDim.x) cp_async_one(A + L.pos_c[j], psi + j);
+    for_cells<4>(p.a_c + threadIdx.x, p.b_c, blockDim.x, L.pos_c, [&](int j, int at) { cp_async_one(A + at, psi + j); });
+    // a cell a lane here: the copies of a cell's values share its place and hit
+    // L1 after the first (values across lanes: K1 0.51 -> 0.57 ms on 128 x 48^3)
     const T *pf = psi + L.nvctr_c;
-#pragma unroll 4
-    for (int j = p.a_f + threadIdx.x; j < p.b_f; j += blockDim.x) {
-        T *a = A + L.pos_f[j];
+    for_cells<4>(p.a_f + threadIdx.x, p.b_f, blockDim.x, L.pos_f, [&](int j, int at) {
         const T *src = pf + 7 * (size_t)j;
 #pragma unroll
         for (int c = 1; c <= 7; ++c)
-            if (fs3(c) == S3) cp_async_one(a + comp_ofs(c, p.H1, p.wrow), src + c - 1);
-    }
+            if (fs3(c) == S3) cp_async_one(A + at + comp_ofs(c, p.H1, p.wrow), src + c - 1);
+    });
 }
 
 template <class T>
@@ -391,11 +428,8 @@ __device__ __forceinline__ TO *out_ptr(const OrbDev &o, TO *base)
     return o.out_ptr ? (TO *)o.out_ptr : base + o.psi;
 }
 
-// Resident CTAs per SM the plane kernels are compiled for (plane_ctas_per_sm
-// in wvlh_internal.h): FP32 CTAs of 1024, 512, 384, 256 or 128 threads at 64,
-// 64, 56, 64, 64 registers; FP64 CTAs of 512, 256 or 128 threads at up to 128
-// registers; the 384-thread FP64 and the persistent variants take what their
-// registers need.
+// Resident CTAs per SM the plane kernels are compiled for (plane_ctas_per_sm in
+// wvlh_internal.h); the persistent variants take what their registers need.
 __host__ __device__ constexpr int plane_min_blocks(bool fp32, bool persist, int nt)
 {
     return persist ? 1 : plane_ctas_per_sm(fp32, nt);
@@ -417,63 +451,50 @@ template <class T> struct CgIo {
 
 // The CG direction of wavelet plane kz, formed while it is gathered: every
 // coefficient gets v = r (first) or beta d + r, written back to d and into A
-// scaled by D^-1/2.  A thread loads the d and r values of two cells before it
-// stores any (a store to d would hold back the next cell's loads).
+// scaled by D^-1/2.  A thread loads d and r of two cells (four coarse values)
+// before it stores any: a store to d would hold back the next cell's loads.
 template <class T, int S3>
 __device__ __forceinline__ void cg_dir_plane_s(T *A, int pitch, const LrDev &L, int i3, T *d, const T *__restrict__ r,
                                                T beta, bool first, const T *sc)
 {
     const PlaneCells p(L, pitch, i3, !S3);
-    constexpr int K = 2, NC = S3 ? 4 : 3, C0 = S3 ? 4 : 1;
-    const int nt = blockDim.x;
-    for (int j0 = p.a_c + threadIdx.x; j0 < p.b_c; j0 += 4 * nt) {
-        T v[4];
-        int at[4];
+    // NC values of each of K cells, a cell's at index idx(j) + c, place at + ofs[c]
+    auto run = [&](auto kc, auto nc, int j0, int end, const int *__restrict__ pos, int stride, T *dv, const T *__restrict__ rv,
+                   int c0) {
+        constexpr int K = decltype(kc)::value, NC = decltype(nc)::value;
+        const int step = blockDim.x;
+        for (; j0 < end; j0 += K * step) {
+            T v[K][NC];
+            int at[K];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const int j = j0 + k * nt;
-            if (j < p.b_c) {
-                at[k] = L.pos_c[j];
-                v[k] = first ? r[j] : fma(beta, d[j], r[j]);
+            for (int k = 0; k < K; ++k) {
+                const int j = j0 + k * step;
+                if (j < end) {
+                    at[k] = __ldg(pos + j);
+                    const size_t i = (size_t)stride * j;
+#pragma unroll
+                    for (int c = 0; c < NC; ++c) v[k][c] = first ? rv[i + c] : fma(beta, dv[i + c], rv[i + c]);
+                }
             }
-        }
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const int j = j0 + k * nt;
-            if (j < p.b_c) {
-                d[j] = v[k];
-                A[at[k]] = v[k] * sc[0];
-            }
-        }
-    }
-    T *df = d + L.nvctr_c;
-    const T *rf = r + L.nvctr_c;
-    for (int j0 = p.a_f + threadIdx.x; j0 < p.b_f; j0 += K * nt) {
-        T v[K][NC];
-        int at[K];
+            for (int k = 0; k < K; ++k) {
+                const int j = j0 + k * step;
+                if (j < end) {
+                    const size_t i = (size_t)stride * j;
 #pragma unroll
-        for (int k = 0; k < K; ++k) {
-            const int j = j0 + k * nt;
-            if (j < p.b_f) {
-                at[k] = L.pos_f[j];
-                const size_t i = 7 * (size_t)j + C0 - 1;
-#pragma unroll
-                for (int c = 0; c < NC; ++c) v[k][c] = first ? rf[i + c] : fma(beta, df[i + c], rf[i + c]);
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < K; ++k) {
-            const int j = j0 + k * nt;
-            if (j < p.b_f) {
-                const size_t i = 7 * (size_t)j + C0 - 1;
-#pragma unroll
-                for (int c = 0; c < NC; ++c) {
-                    df[i + c] = v[k][c];
-                    A[at[k] + comp_ofs(C0 + c, p.H1, p.wrow)] = v[k][c] * sc[C0 + c];
+                    for (int c = 0; c < NC; ++c) {
+                        dv[i + c] = v[k][c];
+                        A[at[k] + comp_ofs(c0 + c, p.H1, p.wrow)] = v[k][c] * sc[c0 + c];
+                    }
                 }
             }
         }
-    }
+    };
+    using std::integral_constant;
+    run(integral_constant<int, 4>(), integral_constant<int, 1>(), p.a_c + threadIdx.x, p.b_c, L.pos_c, 1, d, r, 0);
+    constexpr int NC = S3 ? 4 : 3, C0 = S3 ? 4 : 1;
+    run(integral_constant<int, 2>(), integral_constant<int, NC>(), p.a_f + threadIdx.x, p.b_f, L.pos_f, 7,
+        d + L.nvctr_c + C0 - 1, r + L.nvctr_c + C0 - 1, C0);
 }
 
 // ---------------------------------------------------------------------------
@@ -498,6 +519,7 @@ __device__ __forceinline__ void k1_item(const LrDev *__restrict__ lrs, const Orb
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     using U = typename ColUnit<T>::U;
+    constexpr int kSeg = plane_seg(sizeof(T) == 4);
     {
         const int oi = find_owner(pre, norb, it);   // item = (orbital, wavelet plane kz)
         const int kz = it - pre[oi];
@@ -544,7 +566,7 @@ __device__ __forceinline__ void k1_item(const LrDev *__restrict__ lrs, const Orb
         for_items((d.I1 + U::n - 1) / U::n, (npair + kSeg - 1) / kSeg, [&](int u, int s) {
             const int u0 = s * kSeg;
             typename U::V acc[2 * kSeg];
-            col_b<U, kSeg>(acc, B + u * U::n, pitch, d.N2, d.N2, d.p2, u0);
+            col_b<U, kSeg>(acc, B, u * U::n, pitch, d.N2, d.N2, d.p2, u0);
             T *o = q + (size_t)(2 * u0) * d.IP1 + u * U::n;
 #pragma unroll
             for (int t = 0; t < 2 * kSeg; ++t)
@@ -584,7 +606,8 @@ __global__ void __launch_bounds__(NT, plane_min_blocks(sizeof(T) == 4, PERSIST, 
 // of one z segment.  Chain 0 keeps the tile and its real-space form in shared
 // memory, chain 1 the tile alone; both write their outputs straight to global
 // memory, lanes on neighbouring columns.
-// NT threads per CTA: 256, or for FP32 320 / 384.
+// At most NT threads per CTA (256, or for FP32 320 / 384), as many as share the
+// tile's segments evenly over its rounds (z_block).
 __host__ __device__ constexpr int z_min_blocks(bool fp32, int nt) { return fp32 ? (nt > 256 ? 2 : 3) : 2; }
 
 template <class T, class TV, bool ALLPER, int CHAIN, int NT = kZThreads>
@@ -604,8 +627,8 @@ __global__ void __launch_bounds__(NT, z_min_blocks(sizeof(T) == 4, NT)) k2_zpenc
     // the G1 x G2 plane of D, row-major; pre is the chain's own prefix table
     constexpr int chain = CHAIN == 2 ? 1 : CHAIN;
     constexpr bool EN = CHAIN != 2;
-    constexpr int NU = TC / U::n, DS = NT / NU;   // column units, segments in flight
-    static_assert(NT % NU == 0, "whole segments per round");
+    constexpr int NU = TC / U::n;       // column units
+    const int DS = blockDim.x / NU;     // segments in flight (blockDim.x: whole ones)
     const int oi = find_owner(pre, norb, blockIdx.x);
     const int jj = blockIdx.x - pre[oi];   // tile index, also the energy slot
     const OrbDev o = orbs[oi];
@@ -651,7 +674,8 @@ __global__ void __launch_bounds__(NT, z_min_blocks(sizeof(T) == 4, NT)) k2_zpenc
     } else {
         // column pairs (x, x + 1) of one tile row: the rows have an even pitch
         // and start on a pair
-        constexpr int TP = TC / 2, ZP = NT / TP;
+        constexpr int TP = TC / 2;
+        const int ZP = blockDim.x / TP;
         const int pc = 2 * (threadIdx.x % TP);
         const int xp = x0 + (pc % TX), yp = y0 + (pc / TX);
         const bool pin = xp < W && yp < H;
@@ -678,12 +702,12 @@ __global__ void __launch_bounds__(NT, z_min_blocks(sizeof(T) == 4, NT)) k2_zpenc
         pv += in0 ? (size_t)yu * W + xu : 0;
         T ep = T(0);
         const int npair = d.p3 ? d.N3 : d.N3 + 15;
-        for (int s = sg; s * kSeg < npair; s += DS) {
-            const int z0 = 2 * s * kSeg;
+        for (int s = sg; s * kSegZ < npair; s += DS) {
+            const int z0 = 2 * s * kSegZ;
             // the potential's points are on their way while the filter runs
-            V v[2 * kSeg], acc[2 * kSeg];
+            V v[2 * kSegZ], acc[2 * kSegZ];
 #pragma unroll
-            for (int t = 0; t < 2 * kSeg; ++t) {
+            for (int t = 0; t < 2 * kSegZ; ++t) {
                 v[t] = U::zero();
                 if (z0 + t < d.I3 && in0) {
                     const TV *a = pv + (size_t)(z0 + t) * vplane;
@@ -699,10 +723,10 @@ __global__ void __launch_bounds__(NT, z_min_blocks(sizeof(T) == 4, NT)) k2_zpenc
                     }
                 }
             }
-            col_b<U, kSeg>(acc, A + uc, TC, d.N3, d.N3, d.p3, s * kSeg);
+            col_b<U, kSegZ>(acc, A, uc, TC, d.N3, d.N3, d.p3, s * kSegZ);
             V es = U::zero();
 #pragma unroll
-            for (int t = 0; t < 2 * kSeg; ++t) {
+            for (int t = 0; t < 2 * kSegZ; ++t) {
                 if (z0 + t < d.I3) {
                     const V w = U::mulv(v[t], acc[t]);
                     es = U::fmav(w, acc[t], es);
@@ -713,13 +737,13 @@ __global__ void __launch_bounds__(NT, z_min_blocks(sizeof(T) == 4, NT)) k2_zpenc
         }
         e = (double)ep;
         __syncthreads();
-        for (int s = sg; s * kSeg < d.N3; s += DS) {
-            const int i0 = s * kSeg;
-            V c[kSeg], w[kSeg];
-            col_bt<U, kSeg>(c, w, B + uc, TC, d.I3, d.p3, i0);
+        for (int s = sg; s * kSegZ < d.N3; s += DS) {
+            const int i0 = s * kSegZ;
+            V c[kSegZ], w[kSegZ];
+            col_bt<U, kSegZ>(c, w, B, uc, TC, d.I3, d.p3, i0);
             if (in0) {
 #pragma unroll
-                for (int t = 0; t < kSeg; ++t)
+                for (int t = 0; t < kSegZ; ++t)
                     if (i0 + t < d.N3) {
                         *reinterpret_cast<V *>(gz + (size_t)(i0 + t) * plane) = c[t];
                         *reinterpret_cast<V *>(gz + (size_t)(d.N3 + i0 + t) * plane) = w[t];
@@ -727,15 +751,14 @@ __global__ void __launch_bounds__(NT, z_min_blocks(sizeof(T) == 4, NT)) k2_zpenc
             }
         }
     } else {
-        const double scale = -0.5 / (L.hgrid[2] * L.hgrid[2]);
-        for (int s = sg; s * kSeg < d.N3; s += DS) {
-            const int i0 = s * kSeg;
-            V c[kSeg], w[kSeg], es = U::zero();
-            Lags<U> lag;
-            col_t<U, kSeg, EN>(c, w, A + uc, TC, d.N3, d.N3, d.p3, i0, lag);
+        const double scale = -0.5 / (L.hgrid[2] * L.hgrid[2] * TNorm<T>::v);
+        for (int s = sg; s * kSegZ < d.N3; s += DS) {
+            const int i0 = s * kSegZ;
+            V c[kSegZ], w[kSegZ], es = U::zero();
+            col_t<U, kSegZ>(c, w, A, uc, TC, d.N3, d.N3, d.p3, i0);
             if (in0) {
 #pragma unroll
-                for (int t = 0; t < kSeg; ++t)
+                for (int t = 0; t < kSegZ; ++t)
                     if (i0 + t < d.N3) {
                         if (EN) {
                             es = U::fmav(c[t], *reinterpret_cast<const V *>(A + (i0 + t) * TC + uc), es);
@@ -744,7 +767,7 @@ __global__ void __launch_bounds__(NT, z_min_blocks(sizeof(T) == 4, NT)) k2_zpenc
                         *reinterpret_cast<V *>(gz + (size_t)(i0 + t) * plane) = U::mul((T)scale, c[t]);
                         *reinterpret_cast<V *>(gz + (size_t)(d.N3 + i0 + t) * plane) = U::mul((T)scale, w[t]);
                     }
-                if (EN) e += ((double)U::sum(es) + (sizeof(T) == 4 ? lag.energy() : 0.0)) * scale;
+                if (EN) e += (double)U::sum(es) * scale;
             }
         }
     }
@@ -768,6 +791,7 @@ __device__ __forceinline__ void k3_item(const LrDev *__restrict__ lrs, const Orb
     extern __shared__ __align__(128) unsigned char smem_raw[];
     using U = typename ColUnit<T>::U;
     using V = typename U::V;
+    constexpr int kSeg = plane_seg(sizeof(T) == 4);
     {
         const int oi = find_owner(pre, norb, it);   // item = (orbital, wavelet plane kz)
         const int kz = it - pre[oi];
@@ -791,7 +815,7 @@ __device__ __forceinline__ void k3_item(const LrDev *__restrict__ lrs, const Orb
             for_items((d.I1 + U::n - 1) / U::n, (d.N2 + kSeg - 1) / kSeg, [&](int u, int s) {
                 const int i0 = s * kSeg;
                 V c[kSeg], w[kSeg];
-                col_bt<U, kSeg>(c, w, A + u * U::n, pitch, d.I2, d.p2, i0);
+                col_bt<U, kSeg>(c, w, A, u * U::n, pitch, d.I2, d.p2, i0);
                 T *b = B + i0 * pitch + u * U::n;
 #pragma unroll
                 for (int t = 0; t < kSeg; ++t)
@@ -806,6 +830,12 @@ __device__ __forceinline__ void k3_item(const LrDev *__restrict__ lrs, const Orb
         }
         if (bslice) load_wavelet<T, false>(B, pitch, d, scratch + o.sP + wofs);
         else load_wavelet<T, true>(B, pitch, d, scratch + o.sP + wofs);
+        // Z2 into A while D is on its way (in the y pass's epilogue its loads
+        // stood at the end of every thread's work: 70 of the kernel's 172 us on
+        // 24 x 48^3, where that pass computes for 26)
+        const T *z2 = scratch + o.sZ + wofs;
+        if (MODE == MODE_PRECOND) load_wavelet<T, true>(A, pitch, d, z2);
+        else add_wavelet(A, pitch, d, z2);
         cp_async_wait_all();
         __syncthreads();
         // e: the kinetic energy partial (MODE_LOCHAM) or <d | A d>
@@ -813,42 +843,22 @@ __device__ __forceinline__ void k3_item(const LrDev *__restrict__ lrs, const Orb
         // W = (c + T) D before its scaling
         constexpr bool EN = MODE != MODE_PRECOND;
         double e = 0.0;
-        const double sx = -0.5 / (L.hgrid[0] * L.hgrid[0]);
-        const double sy = -0.5 / (L.hgrid[1] * L.hgrid[1]);
-        row_t<T, kSeg, EN, EN>(B, A, d.G2, pitch, d.N1, d.H1, d.p1, sx, cshift, &e);
+        const double sx = -0.5 / (L.hgrid[0] * L.hgrid[0] * TNorm<T>::v);
+        const double sy = -0.5 / (L.hgrid[1] * L.hgrid[1] * TNorm<T>::v);
+        row_t<T, kSeg, !EN, EN>(B, A, d.G2, pitch, d.N1, d.H1, d.p1, sx, cshift, &e);   // += T_x D (+ c D)
         __syncthreads();
-        // + T_y D + Z2, the plane's columns
-        const T *z2 = scratch + o.sZ + wofs;
-        const bool odd = d.N1 & 1;
+        // + T_y D, the plane's columns (the pad columns of odd rows are zero in D)
         for_items(2 * d.H1 / U::n, (d.N2 + kSeg - 1) / kSeg, [&](int u, int sg) {
             const int i0 = sg * kSeg, col = u * U::n;
-            // this unit's columns in the dense Z2 plane (none for a pad column)
-            const int g0 = col < d.H1 ? col : col - d.H1 + d.N1;
-            const bool h0 = col != d.N1 && col != d.H1 + d.N1;
-            const int g1 = col + 1 < d.H1 ? col + 1 : col + 1 - d.H1 + d.N1;
-            const bool h1 = col + 1 != d.N1 && col + 1 != d.H1 + d.N1;
             V s[kSeg], w[kSeg], es = U::zero();
-            Lags<U> lag;
-            col_t<U, kSeg, EN>(s, w, B + col, pitch, d.N2, d.N2, d.p2, i0, lag);
+            col_t<U, kSeg>(s, w, B, col, pitch, d.N2, d.N2, d.p2, i0);
             auto put = [&](int row, V conv) {
-                const T *zr = z2 + (size_t)row * d.G1;
-                V z;
-                if constexpr (U::n == 2) {
-                    if (!odd) {
-                        z = *reinterpret_cast<const V *>(zr + g0);
-                    } else {
-                        z.x = h0 ? zr[g0] : T(0);
-                        z.y = h1 ? zr[g1] : T(0);
-                    }
-                } else {
-                    z = !odd || h0 ? zr[g0] : T(0);
-                }
                 V *a = reinterpret_cast<V *>(A + row * pitch + col);
                 const V x = *reinterpret_cast<const V *>(B + row * pitch + col);
-                const V r = U::fma((T)sy, conv, U::add(*a, z));
+                const V r = U::fma((T)sy, conv, *a);
                 *a = r;
                 if (EN) es = U::fmav(x, conv, es);
-                else if (dotv) U::dot(e, x, r, odd ? h0 : true, odd ? h1 : true);
+                else if (dotv) U::dot(e, x, r);
             };
 #pragma unroll
             for (int t = 0; t < kSeg; ++t)
@@ -856,7 +866,7 @@ __device__ __forceinline__ void k3_item(const LrDev *__restrict__ lrs, const Orb
                     put(i0 + t, s[t]);
                     put(d.N2 + i0 + t, w[t]);
                 }
-            if (EN) e += ((double)U::sum(es) + (sizeof(T) == 4 ? lag.energy() : 0.0)) * sy;
+            if (EN) e += (double)U::sum(es) * sy;
         });
         __syncthreads();
         scatter_plane<T, TO>(A, pitch, L, kz, out_ptr(o, hpsi), accumulate != 0, MODE == MODE_PRECOND ? sc : nullptr);
@@ -867,8 +877,6 @@ __device__ __forceinline__ void k3_item(const LrDev *__restrict__ lrs, const Orb
     }
 }
 
-// FP32: 3 CTAs per SM (56 registers), which the 75 KB of shared memory of a
-// 96^2 plane pair allows; FP64 planes leave room for one CTA anyway
 template <class T, class TO, bool ALLPER, int MODE, bool PERSIST, int NT>
 __global__ void __launch_bounds__(NT, plane_min_blocks(sizeof(T) == 4, PERSIST, NT)) k3_plane_backward(const LrDev *__restrict__ lrs,
                                                                    const OrbDev *__restrict__ orbs,
@@ -918,8 +926,11 @@ static __global__ void k_reduce_energies(const double *__restrict__ part_pot, co
 // ---------------------------------------------------------------------------
 // Density z-kernel: for a tile of ISF columns, loop over the orbitals of one
 // chunk: R = M_z S_z Q, acc += hfac R^2 (FP64), then write the chunk partial.
+// Segments of six points: 256 threads then share the 32 column units of a
+// 48-cell line's eight segments in one round.
+constexpr int kDenSeg = 6;
 template <class T, bool ALLPER, int MAXP>
-__global__ void __launch_bounds__(kZThreads) kd_density(const LrDev *__restrict__ lrs,
+__global__ void __launch_bounds__(kZThreads, MAXP > 32 ? 1 : 2) kd_density(const LrDev *__restrict__ lrs,
                                                         const OrbDev *__restrict__ orbs,
                                                         const int *__restrict__ pre, int nchunk,
                                                         const int *__restrict__ chunk_orb_start,
@@ -965,12 +976,12 @@ __global__ void __launch_bounds__(kZThreads) kd_density(const LrDev *__restrict_
             cp_async_pair_z(A + z * TC + pc, g + (pin ? (size_t)z * plane + pofs : 0), pin);
         cp_async_wait_all();
         __syncthreads();
-        for (int s = threadIdx.x / NU; s * kSeg < npair; s += DS) {
-            typename U::V r[2 * kSeg];
-            col_b<U, kSeg>(r, A + uc, TC, d.N3, d.N3, d.p3, s * kSeg);
+        for (int s = threadIdx.x / NU; s * kDenSeg < npair; s += DS) {
+            typename U::V r[2 * kDenSeg];
+            col_b<U, kDenSeg>(r, A, uc, TC, d.N3, d.N3, d.p3, s * kDenSeg);
 #pragma unroll
-            for (int t = 0; t < 2 * kSeg; ++t)
-                if (2 * s * kSeg + t < d.I3) *reinterpret_cast<typename U::V *>(B + (2 * s * kSeg + t) * TC + uc) = r[t];
+            for (int t = 0; t < 2 * kDenSeg; ++t)
+                if (2 * s * kDenSeg + t < d.I3) *reinterpret_cast<typename U::V *>(B + (2 * s * kDenSeg + t) * TC + uc) = r[t];
         }
         __syncthreads();
         const double hf = hfac[orb];
@@ -1198,28 +1209,27 @@ static PlaneCfg plane_cfg(const Plan &p, int fp, int nwork)
     return c;
 }
 
+// the variant compiled for the smallest size that takes pc.threads
 template <class T, class TI, bool ALLPER, int MODE>
-static auto k1_for(const PlaneCfg &pc) -> decltype(&k1_plane_forward<T, TI, ALLPER, MODE, false, kPlaneThreads>)
+static auto k1_for(const PlaneCfg &pc) -> decltype(&k1_plane_forward<T, TI, ALLPER, MODE, true, kPlaneThreads>)
 {
     if (pc.global_b) return k1_plane_forward<T, TI, ALLPER, MODE, true, kPlaneThreads>;
-    if constexpr (sizeof(T) == 4)
-        if (pc.threads == 1024) return k1_plane_forward<T, TI, ALLPER, MODE, false, 1024>;
-    if (pc.threads == 512) return k1_plane_forward<T, TI, ALLPER, MODE, false, 512>;
-    if (pc.threads == 128) return k1_plane_forward<T, TI, ALLPER, MODE, false, 128>;
-    if (pc.threads == 256) return k1_plane_forward<T, TI, ALLPER, MODE, false, 256>;
-    return k1_plane_forward<T, TI, ALLPER, MODE, false, kPlaneThreads>;
+    if (pc.threads <= kPlaneSizes[4]) return k1_plane_forward<T, TI, ALLPER, MODE, false, kPlaneSizes[4]>;
+    if (pc.threads <= kPlaneSizes[3]) return k1_plane_forward<T, TI, ALLPER, MODE, false, kPlaneSizes[3]>;
+    if (pc.threads <= kPlaneSizes[2]) return k1_plane_forward<T, TI, ALLPER, MODE, false, kPlaneSizes[2]>;
+    if (pc.threads <= kPlaneSizes[1]) return k1_plane_forward<T, TI, ALLPER, MODE, false, kPlaneSizes[1]>;
+    return k1_plane_forward<T, TI, ALLPER, MODE, false, kPlaneSizes[0]>;
 }
 
 template <class T, class TO, bool ALLPER, int MODE>
-static auto k3_for(const PlaneCfg &pc) -> decltype(&k3_plane_backward<T, TO, ALLPER, MODE, false, kPlaneThreads>)
+static auto k3_for(const PlaneCfg &pc) -> decltype(&k3_plane_backward<T, TO, ALLPER, MODE, true, kPlaneThreads>)
 {
     if (pc.global_b) return k3_plane_backward<T, TO, ALLPER, MODE, true, kPlaneThreads>;
-    if constexpr (sizeof(T) == 4)
-        if (pc.threads == 1024) return k3_plane_backward<T, TO, ALLPER, MODE, false, 1024>;
-    if (pc.threads == 512) return k3_plane_backward<T, TO, ALLPER, MODE, false, 512>;
-    if (pc.threads == 128) return k3_plane_backward<T, TO, ALLPER, MODE, false, 128>;
-    if (pc.threads == 256) return k3_plane_backward<T, TO, ALLPER, MODE, false, 256>;
-    return k3_plane_backward<T, TO, ALLPER, MODE, false, kPlaneThreads>;
+    if (pc.threads <= kPlaneSizes[4]) return k3_plane_backward<T, TO, ALLPER, MODE, false, kPlaneSizes[4]>;
+    if (pc.threads <= kPlaneSizes[3]) return k3_plane_backward<T, TO, ALLPER, MODE, false, kPlaneSizes[3]>;
+    if (pc.threads <= kPlaneSizes[2]) return k3_plane_backward<T, TO, ALLPER, MODE, false, kPlaneSizes[2]>;
+    if (pc.threads <= kPlaneSizes[1]) return k3_plane_backward<T, TO, ALLPER, MODE, false, kPlaneSizes[1]>;
+    return k3_plane_backward<T, TO, ALLPER, MODE, false, kPlaneSizes[0]>;
 }
 
 // TMA maps of the z kernel's tiles: when every orbital of the batch lies in
@@ -1268,7 +1278,15 @@ static cudaError_t run_k3(const Plan &p, const PlaneCfg &pc, const T *scratch, T
     return cudaSuccess;
 }
 
-// K2 launch with the block size zt (FP32: 256, 320 or 384; FP64: 256)
+// threads of a z-kernel CTA compiled for nt: the tile's segments (its longest
+// line's) in equal rounds
+static int z_block(bool fp32, int segs, int nt)
+{
+    const int nu = TC / (fp32 ? 2 : 1), most = nt / nu, rounds = (segs + most - 1) / most;
+    return rounds > 0 ? nu * ((segs + rounds - 1) / rounds) : nt;
+}
+
+// K2 launch with the kernel compiled for zt threads (FP32: 256, 320 or 384; FP64: 256)
 template <class T, class TV, bool ALLPER, int CHAIN>
 static cudaError_t run_k2(int zt, int nwork, size_t sm2, const Plan &p, const int *pre, const TV *pot, T *scratch,
                           double *part_pot, double *part_kin, int part_stride, const CUtensorMap &m_in, int tma,
@@ -1282,6 +1300,7 @@ static cudaError_t run_k2(int zt, int nwork, size_t sm2, const Plan &p, const in
     } else {
         zt = kZThreads;
     }
+    zt = z_block(sizeof(T) == 4, CHAIN == 0 ? p.z_segs0 : p.z_segs1, zt);
     cudaError_t err;
     if ((err = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm2))) return err;
     k<<<nwork, zt, sm2, st>>>(p.d_lr, p.d_orb, pre, p.norb, pot, scratch, part_pot, part_kin, part_stride, m_in,

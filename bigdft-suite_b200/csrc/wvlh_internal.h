@@ -11,62 +11,78 @@ namespace wvlh {
 // z-kernel tile: TX_ consecutive x by TY_ rows of columns
 constexpr int TX_ = 32;
 constexpr int TY_ = 2;
-// block sizes of the plane kernels (K1, K3) and of the z-pencil kernel (K2);
-// 384 threads give 3 line-segment items per thread on 96-point planes
+// Wavelet points of a line segment one thread takes in the fused kernels'
+// passes: eight, 16 accumulators in flight, as boxes are mostly multiples of
+// eight; six in the FP32 plane kernels, which then fill 384 threads on a 96 x 96
+// plane (K1 and K3 of 128 orbitals 0.51 + 1.19 ms, with eight 0.57 + 1.24).  The
+// FP64 plane kernels (32^3: K3 0.85 -> 0.68 ms) and the z kernel (40^3 FP32 0.60
+// -> 0.49 ms) gain from eight: fewer window loads an output.
+constexpr int kSegZ = 8;
+__host__ __device__ constexpr int plane_seg(bool fp32) { return fp32 ? 6 : 8; }
+// block size of the persistent plane kernels
 constexpr int kPlaneThreads = 384;
 
-// CTAs per SM the plane kernels are compiled for (register budget): FP32
-// 1024 / 512 / 384 / 256 / 128 threads -> 1 / 2 / 3 / 4 / 8; FP64 (no 1024)
-// 512 / 384 / 256 / 128 -> 1 / 1 / 2 / 4.
+// The plane kernels (K1, K3) run with any block size; they are compiled for
+// these bounds, at 65536 / (bound x CTAs per SM) registers a thread: FP32 56,
+// 56, 72, 64, 64; FP64 112, 168, 112, 112, 128.  Two planes of a 96 x 96 box
+// leave room for three FP32 CTAs or one FP64 CTA.
+constexpr int kPlaneSizes[5] = {576, 384, 288, 192, 128};
 __host__ __device__ constexpr int plane_ctas_per_sm(bool fp32, int nt)
 {
-    return fp32 ? (nt >= 1024 ? 1 : nt >= 512 ? 2 : nt >= 384 ? 3 : nt >= 256 ? 4 : 8)
-                : (nt >= 384 ? 1 : nt >= 256 ? 2 : 4);
+    return fp32 ? (nt > 384 ? 2 : nt > 192 ? 3 : nt > 128 ? 5 : 8) : (nt > 288 ? 1 : nt > 192 ? 2 : nt > 128 ? 3 : 4);
 }
 
-// CTA size of the plane kernels, chosen per batch by a small occupancy model.
-// A pass over rows has `rows` lines, one over columns len lines (two FP32
-// columns or one FP64 column a thread), each cut into segments of 12 points;
-// with nt threads a pass of n items takes ceil(n / nt) rounds, so the busy
-// fraction is the two passes' items over their rounds times nt (a column item
-// of two FP32 columns weighs two); the SM holds as many CTAs as registers (the
-// compiled count above), shared memory and threads allow.  The expected rate
-// is busy x resident threads x ctas / (ctas + 1/2) — the last factor because
-// a CTA's barrier waits are covered only by the other resident CTAs; each
-// orbital's planes weigh by their work, and the size with the least total cost
-// wins (a larger CTA on a tie).
+// Block size of the plane kernels, chosen per batch by a small occupancy model.
+// A pass over rows has `rows` lines, one over columns `len` lines (two FP32
+// columns or one FP64 column a thread), each cut into segments of plane_seg
+// wavelet points (twice as many points of a line); with nt threads a pass of n
+// items takes ceil(n / nt) rounds, so the busy fraction is the two passes'
+// items over their rounds times nt (a column item of two FP32 columns weighs
+// two); the SM holds as many CTAs as registers (the compiled count above),
+// shared memory and threads allow.  The expected rate is busy x resident
+// threads x ctas / (ctas + 1/2) -- the last factor because a CTA's barrier
+// waits are covered only by the other resident CTAs; each orbital's planes
+// weigh by their work, and the size with the least total cost wins.
 struct PlaneShape {
     long long rows, len, smem_bytes, weight;
 };
-inline int choose_plane_threads(const std::vector<PlaneShape> &shapes, bool fp32)
+inline double plane_cost(const std::vector<PlaneShape> &shapes, bool fp32, int nt)
 {
-    const int cand32[5] = {1024, 512, kPlaneThreads, 256, 128};
-    const int cand64[4] = {512, kPlaneThreads, 256, 128};
-    const int *cand = fp32 ? cand32 : cand64;
-    const int ncand = fp32 ? 5 : 4;
-    const long long seg = 12, cu = fp32 ? 2 : 1;
+    const long long seg = 2 * plane_seg(fp32), cu = fp32 ? 2 : 1;
+    double cost = 0.0;
+    for (const PlaneShape &s : shapes) {
+        const long long ri = s.rows * ((s.len + seg - 1) / seg);
+        const long long ci = (s.len + cu - 1) / cu * ((s.rows + seg - 1) / seg);
+        const long long rounds = (ri + nt - 1) / nt + cu * ((ci + nt - 1) / nt);
+        const double busy = (double)(ri + cu * ci) / (double)(rounds * nt);
+        const long long by_regs = plane_ctas_per_sm(fp32, nt);
+        const long long by_smem = (227LL * 1024) / (s.smem_bytes + 1024);
+        long long ctas = by_regs < by_smem ? by_regs : by_smem;
+        if (ctas < 1) ctas = 1;
+        cost += (double)s.weight / (busy * (double)ctas * nt * ((double)ctas / ((double)ctas + 0.5)));
+    }
+    return cost;
+}
+// the best block size of each compiled bound (those above the next smaller
+// bound), and the best of all
+inline int choose_plane_threads(const std::vector<PlaneShape> &shapes, bool fp32, int *cand = nullptr)
+{
     double best = 0.0;
     int pick = 0;
-    for (int k = 0; k < ncand; ++k) {
-        const int nt = cand[k];
-        double cost = 0.0;
-        for (const PlaneShape &s : shapes) {
-            const long long ri = s.rows * ((s.len + seg - 1) / seg);
-            const long long ci = (s.len + cu - 1) / cu * ((s.rows + seg - 1) / seg);
-            const long long rounds = (ri + nt - 1) / nt + cu * ((ci + nt - 1) / nt);
-            const double busy = (double)(ri + cu * ci) / (double)(rounds * nt);
-            const long long by_regs = plane_ctas_per_sm(fp32, nt);
-            const long long by_smem = (227LL * 1024) / (s.smem_bytes + 1024);
-            const long long by_threads = 2048 / nt;
-            long long ctas = by_regs < by_smem ? by_regs : by_smem;
-            ctas = ctas < by_threads ? ctas : by_threads;
-            if (ctas < 1) ctas = 1;
-            const double rate = busy * (double)ctas * nt * ((double)ctas / ((double)ctas + 0.5));
-            cost += (double)s.weight / rate;
+    for (int k = 0; k < 5; ++k) {
+        double bk = 0.0;
+        int nk = 0;
+        for (int nt = kPlaneSizes[k]; nt > (k < 4 ? kPlaneSizes[k + 1] : 32); nt -= 32) {
+            const double c = plane_cost(shapes, fp32, nt);
+            if (!nk || c < bk * 0.999) {
+                bk = c;
+                nk = nt;
+            }
         }
-        if (pick == 0 || cost < best * 0.999) {
-            best = cost;
-            pick = nt;
+        if (cand) cand[k] = nk;
+        if (!pick || bk < best * 0.999) {
+            best = bk;
+            pick = nk;
         }
     }
     return pick;
@@ -163,7 +179,9 @@ struct Plan {
     long long planeB_elems = 0;    // elements of buffer B (a plane or a transposed plane)
     int plane_threads[2] = {kPlaneThreads, kPlaneThreads};   // plane-kernel CTA size (float, double)
     int plane_threads_pre[2] = {kPlaneThreads, kPlaneThreads};   // the same for the preconditioner operator
-    int z_threads[2] = {kZThreads, kZThreads};       // z-kernel CTA size (FP32: 256, 320 or 384)
+    int plane_cand[2][5] = {};                       // the sizes that the autotuner measures
+    int z_segs0 = 1, z_segs1 = 1;                    // segments of the longest z line (chain 0, chain 1)
+    int z_threads[2] = {kZThreads, kZThreads};       // z-kernel CTA bound (FP32: 256, 320 or 384)
     int z_threads_pre[2] = {kZThreads, kZThreads};   // the same for the preconditioner operator
     size_t smem2[2] = {0, 0};
     int pitch_max = 0, rows_max = 0, zlen_max = 0;

@@ -30,9 +30,11 @@
 // largest taps of 3.6 and 24.9: under a hundredth of one rounding of the sum.
 //
 // FP32 energies: a tap c rounded to FP32 is off by lo = c - fl(c), the same way
-// for every output.  E_kin = <x | T x> is corrected for the taps whose residual
-// matters (a(0..2) and e(0..1), up to 8e-7; the rest stay below 3e-8) through
-// the line's own lag sums C(l) = sum_i x(i) x(i-l): lo(0) C(0) + 2 sum lo(l) C(l).
+// for every output, and E_kin = <x | T x> by lo(l) sum_i x(i) x(i+l).  The FP32
+// taps of T are kept times kTNorm (the scale -1/(2 h^2) divides by it), a factor
+// found by search so that all the large taps round to within 7e-9 of
+// themselves (unscaled: e(0) by 8e-7, a(1), e(1) by 1e-7): under 4e-8 Ha per
+// axis on a normalised orbital at h = 0.45, with nothing to compute for it.
 // B's residuals move |r|^2 by 2e-9 of itself per axis, below the rounding of r.
 #pragma once
 #include <cuda_runtime.h>
@@ -76,8 +78,7 @@ __device__ __forceinline__ constexpr double t_tap(int o, int i, int l)
     return al > 14 ? 0.0 : o == i ? (o ? e[al] : a[al]) : (o ? c[l + 14] : c[14 - l]);
 }
 template <class T> struct TReach { static constexpr int v = sizeof(T) == 4 ? 11 : 13; };
-// rounding residual of a tap in FP32 (the energy's lag corrections)
-__device__ __forceinline__ constexpr double tap_lo(double c) { return c - (double)(float)c; }
+template <class T> struct TNorm { static constexpr double v = sizeof(T) == 4 ? 1.9474363232066856 : 1.0; };
 
 // ---------------------------------------------------------------- units
 // What one thread carries of a point: a column pass takes 8 bytes of a row of
@@ -100,14 +101,13 @@ struct U2f {
     static __device__ __forceinline__ V fmav(V c, V x, V a) { return __ffma2_rn(c, x, a); }
     static __device__ __forceinline__ V mul(float c, V x) { return __fmul2_rn(make_float2(c, c), x); }
     static __device__ __forceinline__ V mulv(V c, V x) { return __fmul2_rn(c, x); }
-    static __device__ __forceinline__ V add(V a, V b) { return __fadd2_rn(a, b); }
     static __device__ __forceinline__ V zero() { return make_float2(0.f, 0.f); }
     static __device__ __forceinline__ float sum(V a) { return a.x + a.y; }
-    // e += x . r in FP64 over the columns that are there
-    static __device__ __forceinline__ void dot(double &e, V x, V r, bool h0, bool h1)
+    // e += x . r in FP64
+    static __device__ __forceinline__ void dot(double &e, V x, V r)
     {
-        if (h0) e = ::fma((double)x.x, (double)r.x, e);
-        if (h1) e = ::fma((double)x.y, (double)r.y, e);
+        e = ::fma((double)x.x, (double)r.x, e);
+        e = ::fma((double)x.y, (double)r.y, e);
     }
 };
 struct U1d {
@@ -118,8 +118,7 @@ struct U1d {
     static __device__ __forceinline__ V fmav(V c, V x, V a) { return ::fma(c, x, a); }
     static __device__ __forceinline__ V mul(double c, V x) { return c * x; }
     static __device__ __forceinline__ V mulv(V c, V x) { return c * x; }
-    static __device__ __forceinline__ V add(V a, V b) { return a + b; }
-    static __device__ __forceinline__ void dot(double &e, V x, V r, bool h0, bool) { if (h0) e = ::fma(x, r, e); }
+    static __device__ __forceinline__ void dot(double &e, V x, V r) { e = ::fma(x, r, e); }
     static __device__ __forceinline__ V zero() { return 0.0; }
     static __device__ __forceinline__ double sum(V a) { return a; }
 };
@@ -137,9 +136,9 @@ template <> struct RowUnit<double> { using U = U1d; };
 // periodic line is walked by a byte offset that returns to its start at the
 // line's end, in one fused add-and-minimum (right for lines shorter than the
 // window): min(u + step, u + step - length), both unsigned, is the first while
-// u + step stays below the length and the second, wrapped, at the end.  Three
-// integer instructions a load; a compare and select per point took nine, and
-// more of the kernels' issue slots than the multiply-adds.
+// u + step stays below the length and the second, wrapped, at the end.  Two
+// integer instructions a load (three for rows); a compare and select per point
+// took nine, and more of the kernels' issue slots than the multiply-adds.
 
 // p0 moved into [0, L) along a periodic line
 __device__ __forceinline__ int wrap_start(int p0, int L)
@@ -157,22 +156,25 @@ template <class V, class T> __device__ __forceinline__ V load_at(const T *in, un
     return *reinterpret_cast<const V *>(reinterpret_cast<const char *>(in) + byte);
 }
 
-// column units: points lie ps elements apart
+// The unit at column `col` of a buffer whose points (rows) lie ps elements
+// apart.  The column's own offset rides in the walker (it is smaller than a
+// step, so the wrap still falls between the line's ends): the base is the same
+// for every thread and a load needs no address add.
 template <class U, int W, class F>
-__device__ __forceinline__ void col_stream(const typename U::T *in, int ps, int p0, int L, int per, F &&f)
+__device__ __forceinline__ void col_stream(const typename U::T *base, int col, int ps, int p0, int L, int per, F &&f)
 {
     using T = typename U::T;
     using V = typename U::V;
     if (per) {
         const unsigned step = ps * (unsigned)sizeof(T), len = L * step;
-        unsigned u = wrap_start(p0, L) * step;
+        unsigned u = wrap_start(p0, L) * step + col * (unsigned)sizeof(T);
 #pragma unroll
         for (int k = 0; k < W; ++k) {
-            f(k, load_at<V>(in, u));
+            f(k, load_at<V>(base, u));
             u = wrap_step(u, step, len);
         }
     } else {
-        const T *b = in + p0 * ps;
+        const T *b = base + col + p0 * ps;
 #pragma unroll
         for (int k = 0; k < W; ++k)
             f(k, (unsigned)(p0 + k) < (unsigned)L ? *reinterpret_cast<const V *>(b + k * ps) : U::zero());
@@ -248,7 +250,7 @@ __device__ __forceinline__ void bt_point(typename U::V (&c)[HS], typename U::V (
         d[t] = U::fma((T)b_tap(1, m), x, d[t]);
     }
 }
-// s[t], w[t] (coarse point i0 + t of T) from x = point i0 - R + k of input half i
+// s[t], w[t] (coarse point i0 + t of TNorm T) from x = point i0 - R + k of input half i
 template <class U, int SEG, int R>
 __device__ __forceinline__ void t_point(typename U::V (&s)[SEG], typename U::V (&w)[SEG], int k, typename U::V x, int i)
 {
@@ -257,41 +259,10 @@ __device__ __forceinline__ void t_point(typename U::V (&s)[SEG], typename U::V (
     for (int t = 0; t < SEG; ++t) {
         const int l = k - R - t;
         if (l < -R || l > R) continue;
-        s[t] = U::fma((T)t_tap(0, i, l), x, s[t]);
-        w[t] = U::fma((T)t_tap(1, i, l), x, w[t]);
+        s[t] = U::fma((T)(TNorm<T>::v * t_tap(0, i, l)), x, s[t]);
+        w[t] = U::fma((T)(TNorm<T>::v * t_tap(1, i, l)), x, w[t]);
     }
 }
-// Lag sums of a segment's own points (FP32 energies): half 0 lags 0..2, half 1
-// lags 0..1.  point() takes the window points in order, k0 = the first of the
-// segment's own.
-template <class U> struct Lags {
-    using V = typename U::V;
-    V h1, h2, c[2][3];
-    __device__ __forceinline__ Lags() : h1(U::zero()), h2(U::zero())
-    {
-#pragma unroll
-        for (int i = 0; i < 2; ++i)
-#pragma unroll
-            for (int l = 0; l < 3; ++l) c[i][l] = U::zero();
-    }
-    __device__ __forceinline__ void point(int half, bool own, V x)
-    {
-        if (own) {
-            c[half][0] = U::fmav(x, x, c[half][0]);
-            c[half][1] = U::fmav(x, h1, c[half][1]);
-            if (half == 0) c[half][2] = U::fmav(x, h2, c[half][2]);
-        }
-        h2 = h1;
-        h1 = x;
-    }
-    __device__ __forceinline__ double energy() const
-    {
-        double e = tap_lo(t_tap(0, 0, 0)) * (double)U::sum(c[0][0]) + tap_lo(t_tap(1, 1, 0)) * (double)U::sum(c[1][0]);
-        e += 2.0 * (tap_lo(t_tap(0, 0, 1)) * (double)U::sum(c[0][1]) + tap_lo(t_tap(0, 0, 2)) * (double)U::sum(c[0][2]) +
-                    tap_lo(t_tap(1, 1, 1)) * (double)U::sum(c[1][1]));
-        return e;
-    }
-};
 template <class U, int n>
 __device__ __forceinline__ void clear(typename U::V (&acc)[n])
 {
@@ -300,35 +271,35 @@ __device__ __forceinline__ void clear(typename U::V (&acc)[n])
 }
 
 // ---------------------------------------------------------------- column passes
-// One segment of one column unit; `in` points at the unit's point 0, points lie
-// ps elements apart, the wavelet half starts at point H.
+// One segment of the column unit at column `col` of buffer `in`; points lie ps
+// elements apart, the wavelet half starts at point H.
 
 // pairs u0 .. u0 + HS - 1 of B's output (free lines: pair u is the points
 // j = 2u - 14, 2u - 13, stored at 2u, 2u + 1)
 template <class U, int HS>
-__device__ __forceinline__ void col_b(typename U::V (&acc)[2 * HS], const typename U::T *in, int ps, int H, int N,
+__device__ __forceinline__ void col_b(typename U::V (&acc)[2 * HS], const typename U::T *in, int col, int ps, int H, int N,
                                       int per, int u0)
 {
     using V = typename U::V;
     const int p0 = u0 - (per ? 8 : 15);
     clear<U>(acc);
-    col_stream<U, HS + 15>(in, ps, p0, N, per, [&](int k, V x) { b_point<U, HS>(acc, k, x, 0); });
-    col_stream<U, HS + 15>(in + H * ps, ps, p0, N, per, [&](int k, V x) { b_point<U, HS>(acc, k, x, 1); });
+    col_stream<U, HS + 15>(in, col, ps, p0, N, per, [&](int k, V x) { b_point<U, HS>(acc, k, x, 0); });
+    col_stream<U, HS + 15>(in + H * ps, col, ps, p0, N, per, [&](int k, V x) { b_point<U, HS>(acc, k, x, 1); });
 }
 // coarse outputs i0 .. i0 + HS - 1 of B^T; L points of the real-space line
 template <class U, int HS>
-__device__ __forceinline__ void col_bt(typename U::V (&c)[HS], typename U::V (&d)[HS], const typename U::T *in, int ps,
+__device__ __forceinline__ void col_bt(typename U::V (&c)[HS], typename U::V (&d)[HS], const typename U::T *in, int col, int ps,
                                        int L, int per, int i0)
 {
     using V = typename U::V;
     clear<U>(c);
     clear<U>(d);
-    col_stream<U, 2 * HS + 29>(in, ps, 2 * i0 - (per ? 14 : 0), L, per, [&](int k, V x) { bt_point<U, HS>(c, d, k, x); });
+    col_stream<U, 2 * HS + 29>(in, col, ps, 2 * i0 - (per ? 14 : 0), L, per, [&](int k, V x) { bt_point<U, HS>(c, d, k, x); });
 }
-// coarse outputs i0 .. i0 + SEG - 1 of T; with EN, lag += the segment's lag sums
-template <class U, int SEG, bool EN>
-__device__ __forceinline__ void col_t(typename U::V (&s)[SEG], typename U::V (&w)[SEG], const typename U::T *in, int ps,
-                                      int H, int N, int per, int i0, Lags<U> &lag)
+// coarse outputs i0 .. i0 + SEG - 1 of TNorm T
+template <class U, int SEG>
+__device__ __forceinline__ void col_t(typename U::V (&s)[SEG], typename U::V (&w)[SEG], const typename U::T *in, int col, int ps,
+                                      int H, int N, int per, int i0)
 {
     using V = typename U::V;
     constexpr int R = TReach<typename U::T>::v, W = SEG + 2 * R;
@@ -336,11 +307,7 @@ __device__ __forceinline__ void col_t(typename U::V (&s)[SEG], typename U::V (&w
     clear<U>(w);
 #pragma unroll
     for (int i = 0; i < 2; ++i)
-        col_stream<U, W>(in + i * H * ps, ps, i0 - R, N, per, [&](int k, V x) {
-            t_point<U, SEG, R>(s, w, k, x, i);
-            if (EN && sizeof(typename U::T) == 4 && k >= R - 2 && k < R + SEG)
-                lag.point(i, k >= R && i0 + k - R < N, x);
-        });
+        col_stream<U, W>(in + i * H * ps, col, ps, i0 - R, N, per, [&](int k, V x) { t_point<U, SEG, R>(s, w, k, x, i); });
 }
 
 // ---------------------------------------------------------------- row passes
@@ -402,9 +369,9 @@ __device__ __forceinline__ void row_bt(const T *src, T *dst, int nrows, int pitc
     });
 }
 
-// dst row = (ACC ? dst row : cshift src row) + scale T src row; EN: *energy +=
-// <src | scale T src> (a segment's terms in T, the segments in FP64)
-template <class T, int SEG, bool ACC, bool EN>
+// dst row += scale TNorm T src row (SHIFT: + cshift src row); EN: *energy +=
+// <src | scale TNorm T src> (a segment's terms in T, the segments in FP64)
+template <class T, int SEG, bool SHIFT, bool EN>
 __device__ __forceinline__ void row_t(const T *src, T *dst, int nrows, int pitch, int N, int H, int per, double scale_d,
                                       T cshift, double *energy)
 {
@@ -420,25 +387,19 @@ __device__ __forceinline__ void row_t(const T *src, T *dst, int nrows, int pitch
         T s[SEG], w[SEG];
         clear<U>(s);
         clear<U>(w);
-        Lags<U> lag;
 #pragma unroll
         for (int i = 0; i < 2; ++i)
-            row_stream<T, W, -R>(in + i * H, i0, N, per, [&](int k, T x) {
-                t_point<U, SEG, R>(s, w, k, x, i);
-                if (EN && sizeof(T) == 4 && k >= R - 2 && k < R + SEG) lag.point(i, k >= R && i0 + k - R < N, x);
-            });
+            row_stream<T, W, -R>(in + i * H, i0, N, per, [&](int k, T x) { t_point<U, SEG, R>(s, w, k, x, i); });
         T es = T(0);
         auto put = [&](int off, const T(&v)[SEG]) {
 #pragma unroll
             for (int t = 0; t < SEG; t += 2)
                 if (i0 + t < N) {
                     const V2 p = *reinterpret_cast<const V2 *>(in + off + i0 + t);
-                    V2 o;
-                    if (ACC) {
-                        o = *reinterpret_cast<const V2 *>(out + off + i0 + t);
-                    } else {
-                        o.x = cshift * p.x;
-                        o.y = cshift * p.y;
+                    V2 o = *reinterpret_cast<const V2 *>(out + off + i0 + t);
+                    if (SHIFT) {
+                        o.x = U::fma(cshift, p.x, o.x);
+                        o.y = U::fma(cshift, p.y, o.y);
                     }
                     if (EN) {
                         es = U::fma(p.x, v[t], es);
@@ -451,7 +412,7 @@ __device__ __forceinline__ void row_t(const T *src, T *dst, int nrows, int pitch
         };
         put(0, s);
         put(H, w);
-        if (EN) e += ((double)es + (sizeof(T) == 4 ? lag.energy() : 0.0)) * scale_d;
+        if (EN) e += (double)es * scale_d;
     });
     if (EN) *energy += e;
 }

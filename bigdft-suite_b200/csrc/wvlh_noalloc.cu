@@ -273,6 +273,8 @@ extern "C" int wvlh_locham_noalloc(int precision, const int n[3], const int peri
     p.smem13[1] = (rows * pitch + usedB) * 8;
     p.smem2[0] = 2 * zl * TX_ * TY_ * 4;
     p.smem2[1] = 2 * zl * TX_ * TY_ * 8;
+    p.z_segs0 = ((per[2] ? N[2] : N[2] + 15) + kSegZ - 1) / kSegZ;
+    p.z_segs1 = (N[2] + kSegZ - 1) / kSegZ;
     for (int f = 0; f < 2; ++f) {
         p.smem_z0[f] = (size_t)(G[2] + I[2]) * TX_ * TY_ * (f ? 8 : 4);
         p.smem_z1[f] = (size_t)G[2] * TX_ * TY_ * (f ? 8 : 4);

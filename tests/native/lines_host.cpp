@@ -20,13 +20,12 @@
 
 using std::max;
 using std::min;
-static struct { int x; } threadIdx = {0}, blockDim = {1};
+static struct { int x; } threadIdx = {0}, blockDim = {1}, blockIdx = {0};
 static void __syncthreads() {}
 static double __shfl_xor_sync(unsigned, double, int) { return 0.0; }
 static unsigned __viaddmin_u32(unsigned a, unsigned b, unsigned c) { return std::min(a + b, c); }
 static float2 __ffma2_rn(float2 a, float2 b, float2 c) { return {std::fma(a.x, b.x, c.x), std::fma(a.y, b.y, c.y)}; }
 static float2 __fmul2_rn(float2 a, float2 b) { return {a.x * b.x, a.y * b.y}; }
-static float2 __fadd2_rn(float2 a, float2 b) { return {a.x + b.x, a.y + b.y}; }
 
 #include "wvlh_lines.cuh"
 
@@ -55,7 +54,7 @@ template <class T> struct Buf {
     }
 };
 
-constexpr int SEG = 6;
+constexpr int SEG = 8;
 
 template <class T> static void rows(int op, int N, int per, int nrows, const double *in, double *out, double *energy)
 {
@@ -69,7 +68,8 @@ template <class T> static void rows(int op, int N, int per, int nrows, const dou
     double e = 0.0;
     if (op == 0) row_b<T, SEG>(a.p, b.p, nrows, pitch, N, H, per);
     else if (op == 1) row_bt<T, SEG>(a.p, b.p, nrows, pitch, I, N, H, per);
-    else row_t<T, SEG, false, true>(a.p, b.p, nrows, pitch, N, H, per, -0.5, T(0.25), &e);
+    else for (int i = 0; i < nrows * pitch; ++i) b.p[i] = T(0);
+    if (op == 2) row_t<T, SEG, true, true>(a.p, b.p, nrows, pitch, N, H, per, -0.5 / TNorm<T>::v, T(0.25), &e);
     for (int r = 0; r < nrows; ++r)
         for (int c = 0; c < nout; ++c) out[r * nout + c] = b.p[r * pitch + (op == 0 ? c : wpos(c))];
     *energy = e;
@@ -89,36 +89,35 @@ template <class T> static void cols(int op, int N, int per, int ncol, const doub
     auto put = [&](int u, int q, V v) {
         const T *e = (const T *)&v;
         for (int k = 0; k < U::n; ++k)
-            if (u * U::n + k < ncol) out[(u * U::n + k) * nout + q] = (double)e[k];
+            if (u * U::n + k < ncol) out[(u * U::n + k) * nout + q] = (double)e[k] / (op == 2 ? TNorm<T>::v : 1.0);
     };
     double e = 0.0;
     for (int u = 0; u * U::n < ncol; ++u) {
-        const T *col = a.p + u * U::n;
+        const int col = u * U::n;
         if (op == 0) {
             const int np = per ? N : N + 15;
             for (int u0 = 0; u0 < np; u0 += SEG) {
                 V acc[2 * SEG];
-                col_b<U, SEG>(acc, col, ps, N, N, per, u0);
+                col_b<U, SEG>(acc, a.p, col, ps, N, N, per, u0);
                 for (int t = 0; t < 2 * SEG; ++t)
                     if (2 * u0 + t < I) put(u, 2 * u0 + t, acc[t]);
             }
         } else {
             for (int i0 = 0; i0 < N; i0 += SEG) {
                 V c[SEG], d[SEG];
-                Lags<U> lag;
-                if (op == 1) col_bt<U, SEG>(c, d, col, ps, I, per, i0);
-                else col_t<U, SEG, true>(c, d, col, ps, N, N, per, i0, lag);
+                if (op == 1) col_bt<U, SEG>(c, d, a.p, col, ps, I, per, i0);
+                else col_t<U, SEG>(c, d, a.p, col, ps, N, N, per, i0);
                 V es = U::zero();
                 for (int t = 0; t < SEG; ++t)
                     if (i0 + t < N) {
                         put(u, i0 + t, c[t]);
                         put(u, N + i0 + t, d[t]);
                         if (op == 2) {
-                            es = U::fmav(c[t], *(const V *)(col + (i0 + t) * ps), es);
-                            es = U::fmav(d[t], *(const V *)(col + (N + i0 + t) * ps), es);
+                            es = U::fmav(c[t], *(const V *)(a.p + col + (i0 + t) * ps), es);
+                            es = U::fmav(d[t], *(const V *)(a.p + col + (N + i0 + t) * ps), es);
                         }
                     }
-                e += (double)U::sum(es) + (sizeof(T) == 4 ? lag.energy() : 0.0);
+                e += (double)U::sum(es) / TNorm<T>::v;
             }
         }
     }
