@@ -1262,7 +1262,7 @@ extern "C" int wvlh_wpdot(wvlh_ctx *c, int precision, const wvlh_region *ra, int
 
 // ---------------------------------------------------------------------------
 // CUDA graph of one packed-batch locham call (the same batch applied at every
-// SCF iteration): the memsets and kernels are captured once and replayed with
+// SCF iteration): the kernels are captured once and replayed with
 // one launch.  The graph owns its scratch, so that later calls on the context
 // (which may grow the context's buffers) cannot move memory under it.
 struct wvlh_graph {

@@ -610,12 +610,12 @@ __global__ void __launch_bounds__(NT, plane_min_blocks(sizeof(T) == 4, PERSIST, 
 // tile's segments evenly over its rounds (z_block).
 __host__ __device__ constexpr int z_min_blocks(bool fp32, int nt) { return fp32 ? (nt > 256 ? 2 : 3) : 2; }
 
-template <class T, class TV, bool ALLPER, int CHAIN, int NT = kZThreads>
-__global__ void __launch_bounds__(NT, z_min_blocks(sizeof(T) == 4, NT)) k2_zpencil(const LrDev *__restrict__ lrs, const OrbDev *__restrict__ orbs,
-                                                        const int *__restrict__ pre, int norb,
-                                                        const TV *__restrict__ pot, T *__restrict__ scratch,
-                                                        double *__restrict__ part_pot, double *__restrict__ part_kin,
-                                                        int part_stride, const __grid_constant__ CUtensorMap tm_in, int tma)
+template <class T, class TV, bool ALLPER, int CHAIN>
+__device__ __forceinline__ void k2_tile(const LrDev *__restrict__ lrs, const OrbDev *__restrict__ orbs,
+                                        const int *__restrict__ pre, int norb, const TV *__restrict__ pot,
+                                        T *__restrict__ scratch, double *__restrict__ part_pot,
+                                        double *__restrict__ part_kin, int part_stride, const CUtensorMap &tm_in, int tma,
+                                        int item)
 {
     // dynamic shared memory only (the tile, chain 0's real-space tile, then the
     // reduction slots and the TMA barrier), so that the tile starts the
@@ -629,8 +629,8 @@ __global__ void __launch_bounds__(NT, z_min_blocks(sizeof(T) == 4, NT)) k2_zpenc
     constexpr bool EN = CHAIN != 2;
     constexpr int NU = TC / U::n;       // column units
     const int DS = blockDim.x / NU;     // segments in flight (blockDim.x: whole ones)
-    const int oi = find_owner(pre, norb, blockIdx.x);
-    const int jj = blockIdx.x - pre[oi];   // tile index, also the energy slot
+    const int oi = find_owner(pre, norb, item);
+    const int jj = item - pre[oi];   // tile index, also the energy slot
     const OrbDev o = orbs[oi];
     const LrDev L = lrs[o.lr];
     const Dims d(L, ALLPER);
@@ -778,6 +778,34 @@ __global__ void __launch_bounds__(NT, z_min_blocks(sizeof(T) == 4, NT)) k2_zpenc
     }
 }
 
+template <class T, class TV, bool ALLPER, int CHAIN, int NT = kZThreads>
+__global__ void __launch_bounds__(NT, z_min_blocks(sizeof(T) == 4, NT))
+    k2_zpencil(const LrDev *__restrict__ lrs, const OrbDev *__restrict__ orbs, const int *__restrict__ pre, int norb,
+               const TV *__restrict__ pot, T *__restrict__ scratch, double *__restrict__ part_pot,
+               double *__restrict__ part_kin, int part_stride, const __grid_constant__ CUtensorMap tm_in, int tma)
+{
+    k2_tile<T, TV, ALLPER, CHAIN>(lrs, orbs, pre, norb, pot, scratch, part_pot, part_kin, part_stride, tm_in, tma,
+                                  blockIdx.x);
+}
+
+// Both chains in one launch, chain 0's n0 tiles first: for calls whose tiles of
+// both chains fit the chip at once, where the second launch's latency would
+// stand alone (one 32^3 orbital: 64 + 64 tiles on 148 SMs).
+template <class T, class TV, bool ALLPER>
+__global__ void __launch_bounds__(kZThreads, 2)
+    k2_both(const LrDev *__restrict__ lrs, const OrbDev *__restrict__ orbs, const int *__restrict__ pre0,
+            const int *__restrict__ pre1, int n0, int norb, const TV *__restrict__ pot, T *__restrict__ scratch,
+            double *__restrict__ part_pot, double *__restrict__ part_kin, int part_stride,
+            const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_p, int okq, int okp)
+{
+    if ((int)blockIdx.x < n0)
+        k2_tile<T, TV, ALLPER, 0>(lrs, orbs, pre0, norb, pot, scratch, part_pot, part_kin, part_stride, tm_q, okq,
+                                  blockIdx.x);
+    else
+        k2_tile<T, TV, ALLPER, 1>(lrs, orbs, pre1, norb, pot, scratch, part_pot, part_kin, part_stride, tm_p, okp,
+                                  blockIdx.x - n0);
+}
+
 // ---------------------------------------------------------------------------
 // K3 (MODE_LOCHAM): Hpsi plane kz = B^T_x B^T_y Z1 + (T_x + T_y) D + Z2
 // K3 (MODE_PRECOND): D^-1/2 [(c + T_x + T_y) D + Z2]
@@ -902,18 +930,26 @@ __global__ void __launch_bounds__(NT, plane_min_blocks(sizeof(T) == 4, PERSIST, 
     }
 }
 
-// fixed-order per-orbital sum of the energy partial slots
-static __global__ void k_reduce_energies(const double *__restrict__ part_pot, const double *__restrict__ part_kin,
+// energy slots of an orbital: one per chain-0 tile (potential); one per chain-1
+// tile, then one per wavelet plane (kinetic)
+__device__ __forceinline__ int pot_slots(const Dims &d) { return ((d.I1 + TX - 1) / TX) * ((d.I2 + TY - 1) / TY); }
+__device__ __forceinline__ int plane_slot0(const Dims &d) { return ((d.G1 + TX - 1) / TX) * ((d.G2 + TY - 1) / TY); }
+
+// fixed-order per-orbital sum of the energy partials, over the slots that the
+// orbital's tiles and planes write (so nothing has to clear the others first:
+// two memsets less in front of every call)
+static __global__ void k_reduce_energies(const LrDev *__restrict__ lrs, const OrbDev *__restrict__ orbs,
+                                  const double *__restrict__ part_pot, const double *__restrict__ part_kin,
                                   int part_stride, int norb, double *__restrict__ ekin, double *__restrict__ epot)
 {
     __shared__ double red[32];
     const int orb = blockIdx.x;
     if (orb >= norb) return;
+    const Dims d(lrs[orbs[orb].lr], false);
+    const int npot = pot_slots(d), nkin = plane_slot0(d) + d.G3;
     double a = 0.0, b = 0.0;
-    for (int i = threadIdx.x; i < part_stride; i += blockDim.x) {
-        a += part_kin[(size_t)orb * part_stride + i];
-        b += part_pot[(size_t)orb * part_stride + i];
-    }
+    for (int i = threadIdx.x; i < nkin; i += blockDim.x) a += part_kin[(size_t)orb * part_stride + i];
+    for (int i = threadIdx.x; i < npot; i += blockDim.x) b += part_pot[(size_t)orb * part_stride + i];
     const double sa = block_sum(a, red);
     __syncthreads();
     const double sb = block_sum(b, red);
@@ -1186,6 +1222,14 @@ __global__ void k_cg_scale(const LrDev *__restrict__ lrs, const OrbDev *__restri
 
 // Launch shape of the plane kernels: two shared-memory planes when they fit,
 // else one shared plane + a global slice per CTA after the batch scratch.
+static int sm_count()
+{
+    int dev = 0, nsm = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    return nsm;
+}
+
 struct PlaneCfg {
     size_t smem = 0;
     int grid = 0;
@@ -1328,25 +1372,32 @@ static cudaError_t launch_locham_bc(const Plan &p, const TIO *psi, const TIO *po
     const size_t sm2 = p.smem_z0[fp] + kZExtra, sm2p = p.smem_z1[fp] + kZExtra;
     T *gtmp = pc.global_b ? scratch + p.scratch_elems : nullptr;
     cudaError_t err;
-    cudaMemsetAsync(part_pot, 0, sizeof(double) * (size_t)p.norb * p.part_stride, st);
-    cudaMemsetAsync(part_kin, 0, sizeof(double) * (size_t)p.norb * p.part_stride, st);
     ZMaps zm;
     zmaps(p, scratch, zm);
     // optional per-kernel timing: ev[0..4] bracket K1, K2, K3 and the reduction
     if (ev) cudaEventRecord(ev[0], st);
     if ((err = run_k1<T, TIO, ALLPER, MODE_LOCHAM>(p, pc, psi, scratch, nullptr, gtmp, st))) return err;
     if (ev) cudaEventRecord(ev[1], st);
-    if ((err = run_k2<T, TIO, ALLPER, 0>(p.z_threads[fp], p.n_work2, sm2, p, p.d_pre2, pot, scratch, part_pot,
-                                         part_kin, p.part_stride, zm.q, zm.okq, st)) ||
-        (err = run_k2<T, TIO, ALLPER, 1>(p.z_threads[fp], p.n_work2p, sm2p, p, p.d_pre2p, pot, scratch, part_pot,
-                                         part_kin, p.part_stride, zm.p, zm.okp, st)))
+    // both chains' tiles in one wave (two CTAs an SM, as k2_both is compiled and
+    // FP64 tiles of 64 cells fit): one launch for the two
+    if (p.n_work2 + p.n_work2p <= 2 * sm_count() && 2 * (sm2 + 1024) <= (size_t)227 * 1024) {
+        auto k = k2_both<T, TIO, ALLPER>;
+        if ((err = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm2))) return err;
+        k<<<p.n_work2 + p.n_work2p, z_block(sizeof(T) == 4, p.z_segs0, kZThreads), sm2, st>>>(
+            p.d_lr, p.d_orb, p.d_pre2, p.d_pre2p, p.n_work2, p.norb, pot, scratch, part_pot, part_kin, p.part_stride,
+            zm.q, zm.p, zm.okq, zm.okp);
+    } else if ((err = run_k2<T, TIO, ALLPER, 0>(p.z_threads[fp], p.n_work2, sm2, p, p.d_pre2, pot, scratch, part_pot,
+                                                part_kin, p.part_stride, zm.q, zm.okq, st)) ||
+               (err = run_k2<T, TIO, ALLPER, 1>(p.z_threads[fp], p.n_work2p, sm2p, p, p.d_pre2p, pot, scratch,
+                                                part_pot, part_kin, p.part_stride, zm.p, zm.okp, st))) {
         return err;
+    }
     if (ev) cudaEventRecord(ev[2], st);
     if ((err = run_k3<T, TIO, ALLPER, MODE_LOCHAM>(p, pc, scratch, hpsi, part_kin, p.part_stride, accumulate, nullptr,
                                                    gtmp, st)))
         return err;
     if (ev) cudaEventRecord(ev[3], st);
-    k_reduce_energies<<<p.norb, 128, 0, st>>>(part_pot, part_kin, p.part_stride, p.norb, ekin, epot);
+    k_reduce_energies<<<p.norb, 128, 0, st>>>(p.d_lr, p.d_orb, part_pot, part_kin, p.part_stride, p.norb, ekin, epot);
     if (ev) cudaEventRecord(ev[4], st);
     return cudaGetLastError();
 }
@@ -1412,7 +1463,7 @@ template cudaError_t launch_locden<double>(const Plan &, const double *, const d
 
 // preconditioner operator y = D^-1/2 A (c + T) S D^-1/2 x for every orbital;
 // cg.dir: x is the CG direction, formed by K1 (see CgIo); dotpart: K3's
-// partials of <x | y> per plane (zeroed here first), or null
+// partials of <x | y> per plane, or null
 template <class T, bool ALLPER>
 static cudaError_t launch_prec_apply_bc(const Plan &p, const T *x, T *y, const double *cprec, T *scratch,
                                         cudaStream_t st, const CgIo<T> &cg, double *dotpart)
@@ -1429,22 +1480,24 @@ static cudaError_t launch_prec_apply_bc(const Plan &p, const T *x, T *y, const d
     if ((err = run_k2<T, T, ALLPER, 2>(p.z_threads_pre[fp], p.n_work2p, sm2, p, p.d_pre2p, (const T *)nullptr, scratch,
                                        nullptr, nullptr, 0, zm.p, zm.okp, st)))
         return err;
-    if (dotpart) cudaMemsetAsync(dotpart, 0, sizeof(double) * (size_t)p.norb * p.part_stride, st);
     if ((err = run_k3<T, T, ALLPER, MODE_PRECOND>(p, pc, scratch, y, dotpart, dotpart ? p.part_stride : 0, 0, cprec,
                                                   gtmp, st, dotpart ? x : nullptr)))
         return err;
     return cudaGetLastError();
 }
 
-// out[o] = the sum of orbital o's stride partial slots: one warp per
-// orbital, lane l summing slots l, l + 32, ... then a fixed shuffle tree
+// out[o] = the sum of orbital o's plane partials (K3's slots): one warp per
+// orbital, lane l summing planes l, l + 32, ... then a fixed shuffle tree
 // (deterministic)
-static __global__ void k_cg_sum_slots(int norb, const double *__restrict__ part, int stride, double *__restrict__ out)
+static __global__ void k_cg_sum_slots(const LrDev *__restrict__ lrs, const OrbDev *__restrict__ orbs, int norb,
+                                      const double *__restrict__ part, int stride, double *__restrict__ out)
 {
     const int o = blockIdx.x;
     if (o >= norb) return;
+    const Dims d(lrs[orbs[o].lr], false);
+    const int k0 = plane_slot0(d);
     double s = 0.0;
-    for (int k = threadIdx.x; k < stride; k += 32) s += part[(size_t)o * stride + k];
+    for (int k = threadIdx.x; k < d.G3; k += 32) s += part[(size_t)o * stride + k0 + k];
     s = warp_sum(s);
     if (threadIdx.x == 0) out[o] = s;
 }
@@ -1471,7 +1524,7 @@ static cudaError_t cg_loop(const Plan &p, int ncong, const double *cprec, T *x, 
     for (int it = 0; it < ncong; ++it) {
         if ((err = apply(dvec, ad, CgIo<T>{dvec, r, rr, rrn, it == 0 ? 1 : 2}, dotpart))) return err;
         if (it > 0) k_copy_scalars<<<sg, 128, 0, st>>>(p.norb, rrn, rr);
-        k_cg_sum_slots<<<p.norb, 32, 0, st>>>(p.norb, dotpart, p.part_stride, dad);
+        k_cg_sum_slots<<<p.norb, 32, 0, st>>>(p.d_lr, p.d_orb, p.norb, dotpart, p.part_stride, dad);
         k_cg_step<T, VEC><<<vg, 256, 0, st>>>(p.d_orb_off, p.d_orb_len, rr, dad, x, dvec, r, ad, part);
         k_cg_sum<<<sg, 128, 0, st>>>(p.norb, part, rrn, hist ? hist + (size_t)(it + 1) * p.norb : nullptr);
     }

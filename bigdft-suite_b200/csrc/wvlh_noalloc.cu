@@ -279,7 +279,7 @@ extern "C" int wvlh_locham_noalloc(int precision, const int n[3], const int peri
         p.smem_z0[f] = (size_t)(G[2] + I[2]) * TX_ * TY_ * (f ? 8 : 4);
         p.smem_z1[f] = (size_t)G[2] * TX_ * TY_ * (f ? 8 : 4);
     }
-    // the energy partials are cleared by the launcher; D, Q/Z1, Z2 are fully
+    // the energy slots that are summed, D, Q/Z1 and Z2 are fully
     // overwritten before they are read, so stale contents of an earlier call
     // never leak into this one
     if (precision == 64)
