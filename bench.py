@@ -860,7 +860,9 @@ def main():
         B = 4
         # kernel I/O (what each kernel reads and writes, intermediates included)
         kio = [3 * B * npt * norb, 4 * B * npt * norb + B * npt, 4 * B * npt * norb, 0]
-        kflops = [128 * npt * norb, 252 * npt * norb, 254 * npt * norb, 0]
+        # multiply-adds of the composed passes: 31 taps a point and axis for the magic filter x
+        # synthesis and its transpose, 46 for the kinetic operator in the wavelet basis
+        kflops = [124 * npt * norb, 216 * npt * norb, 308 * npt * norb, 0]
         dom = max(range(3), key=lambda i: kt[i])
         # algorithmic bytes of the path per launch: 8 values in + 8 values out
         # per coarse cell of each orbital (64 B in FP32) plus the potential once
@@ -870,10 +872,10 @@ def main():
         lib().wvlh_measure_fma_peak(32, 20000, C.byref(tf32))
         ach = alg / (kt[dom] * 1e-3) / 1e9
         # DRAM traffic of each kernel (dram__bytes_read.sum + dram__bytes_write.sum) from ncu
-        # captures of one call over 48 orbitals of this 48^3 FP32 workload, scaled by the orbitals
+        # captures of one call over 24 orbitals of this 48^3 FP32 workload, scaled by the orbitals
         # of this launch (the traffic grows in proportion to them); z kernels: both chains
-        traffic48 = [453.519104e6, 582.610688e6, 656.173312e6]
-        traffic = traffic48[dom] / 48 * norb if (dom < 3 and n == 48) else None
+        traffic24 = [203.877632e6, 246.108288e6, 314.778624e6]
+        traffic = traffic24[dom] / 24 * norb if (dom < 3 and n == 48) else None
         step_s = ms / args.steps * 1e-3
         extras["roofline"] = {"bound": "hbm", "achieved": ach, "peak": hbm, "unit": "GB/s", "frac": ach / hbm,
                               "traffic": traffic, "kernel": names[dom], "peak_source": hbm_src,

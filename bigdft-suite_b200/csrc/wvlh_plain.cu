@@ -55,7 +55,7 @@ __global__ void __launch_bounds__(256) k_pass1d(int n, int ndat, int per, double
     else if (KIND == P_MFT) pass_mf<double, 4, 1>(S, D, g, Lin, Lout);
     else if (KIND == P_MFG) pass_mf<double, 4, 2>(S, D, g, Lin, Lout);
     else if (KIND == P_MFS) pass_mf<double, 4, 3>(S, D, g, Lin, Lout);
-    else pass_kin<double, 4, false>(S, D, g, n, per, scale, 0.0, &e);
+    else pass_kin<double, 4>(S, D, g, n, per, scale, 0.0, &e);
     __syncthreads();
     for (int i = threadIdx.x; i < Lout * JT; i += blockDim.x) {
         const int jj = i / Lout, q = i - jj * Lout;
