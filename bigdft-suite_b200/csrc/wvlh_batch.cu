@@ -245,7 +245,7 @@ static int region_make(int device, const wvlh_locreg &L, wvlh_region **out)
     // a box whose cells are all fine has one table for both key sets
     const bool same = L.nseg_c == L.nseg_f && kgc == kgf;
     const size_t tab = (pk.img.size() + 255) & ~size_t(255);
-    if (cudaMalloc(&r->mem, tab + sizeof(int) * ((size_t)nvc + (same ? 0 : nvf))) != cudaSuccess) {
+    if (cudaMalloc(&r->mem, tab + sizeof(uint16_t) * ((size_t)nvc + (same ? 0 : nvf))) != cudaSuccess) {
         r->mem = nullptr;
         region_free(r);
         return WVLH_ERR_NOMEM;
@@ -255,7 +255,7 @@ static int region_make(int device, const wvlh_locreg &L, wvlh_region **out)
         return WVLH_ERR_CUDA;
     }
     pk.place(r->mem);
-    int *pos = reinterpret_cast<int *>(static_cast<unsigned char *>(r->mem) + tab);
+    uint16_t *pos = reinterpret_cast<uint16_t *>(static_cast<unsigned char *>(r->mem) + tab);
     d.pos_c = pos;
     d.pos_f = same ? pos : pos + nvc;
     const int pitch = plane_pitch(d.N[0], d.per[0]);

@@ -93,13 +93,13 @@ __host__ __device__ __forceinline__ int plane_pitch(int N1, int per1)
 
 // Cell table of one key set (LrDev::pos_c / pos_f): one warp per segment.
 static __global__ void k_cell_places(int N1, int N2, int pitch, int nseg, const int32_t *__restrict__ keyg,
-                                     const int32_t *__restrict__ keyv, int *__restrict__ pos)
+                                     const int32_t *__restrict__ keyv, uint16_t *__restrict__ pos)
 {
     const int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (s >= nseg) return;
     const int i = keyg[2 * s] - 1, len = keyg[2 * s + 1] - i, j = keyv[s] - 1;
     const int line = i / N1, x = i - line * N1, y = line % N2;
-    for (int t = lane; t < len; t += 32) pos[j + t] = y * pitch + x + t;
+    for (int t = lane; t < len; t += 32) pos[j + t] = (uint16_t)(y * pitch + x + t);
 }
 
 template <class T> struct Pair;

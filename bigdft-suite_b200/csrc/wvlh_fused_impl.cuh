@@ -116,7 +116,7 @@ __device__ __forceinline__ int comp_ofs(int c, int H1, int wrow) { return fs1(c)
 // f(j, place of cell j) for j = j0, j0 + step, ... < end, the places of K cells
 // read together: their latency would stand before every copy or store
 template <int K, class F>
-__device__ __forceinline__ void for_cells(int j0, int end, int step, const int *__restrict__ pos, F &&f)
+__device__ __forceinline__ void for_cells(int j0, int end, int step, const uint16_t *__restrict__ pos, F &&f)
 {
     for (; j0 < end; j0 += K * step) {
         int at[K];
@@ -459,7 +459,7 @@ __device__ __forceinline__ void cg_dir_plane_s(T *A, int pitch, const LrDev &L, 
 {
     const PlaneCells p(L, pitch, i3, !S3);
     // NC values of each of K cells, a cell's at index idx(j) + c, place at + ofs[c]
-    auto run = [&](auto kc, auto nc, int j0, int end, const int *__restrict__ pos, int stride, T *dv, const T *__restrict__ rv,
+    auto run = [&](auto kc, auto nc, int j0, int end, const uint16_t *__restrict__ pos, int stride, T *dv, const T *__restrict__ rv,
                    int c0) {
         constexpr int K = decltype(kc)::value, NC = decltype(nc)::value;
         const int step = blockDim.x;

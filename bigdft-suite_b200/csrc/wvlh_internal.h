@@ -91,9 +91,10 @@ constexpr int kZThreads = 256;
 
 // One localisation region (box + compressed-key tables) as seen by kernels.
 // The reference's 1-based keyg/keyv (wavelib/un-compress.f90:896-905) are
-// expanded on upload to one word per cell: pos_c / pos_f[j] is the place of the
+// expanded on upload to 16 bits per cell: pos_c / pos_f[j] is the place of the
 // j-th coarse / fine cell of the compressed vector in a wavelet plane of the
-// plane kernels' shared-memory layout (y * pitch + x).  Keys are sorted, so the
+// plane kernels' shared-memory layout (y * pitch + x; a plane that fits shared
+// memory has fewer than 65536 places, larger boxes are refused at launch).  Keys are sorted, so the
 // cells of one z-plane are consecutive: plane_c / plane_f[i3 .. i3+1] delimit
 // those of coarse plane i3.
 struct LrDev {
@@ -101,8 +102,8 @@ struct LrDev {
     int per[3];
     int nseg_c, nseg_f;
     int nvctr_c, nvctr_f;
-    const int *pos_c;
-    const int *pos_f;
+    const uint16_t *pos_c;
+    const uint16_t *pos_f;
     const int *plane_c;  // N3+1 entries
     const int *plane_f;  // N3+1 entries
     double hgrid[3];     // coarse grid spacing

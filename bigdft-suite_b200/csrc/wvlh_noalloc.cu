@@ -36,7 +36,7 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocBytes];
 // scratch has at least 96 bytes of it per coarse cell (three FP32 planes of
 // eight points), which bounds the cells of either key set.
 constexpr size_t kNoAllocCells = kNoAllocBytes / 96 + 1;
-static __device__ int g_noalloc_cells[2 * kNoAllocCells];
+static __device__ uint16_t g_noalloc_cells[2 * kNoAllocCells];
 
 namespace {
 
@@ -170,7 +170,7 @@ extern "C" int wvlh_locham_noalloc(int precision, const int n[3], const int peri
     // kept for the life of the process (the library does not support a reset
     // of the device, which would reload its module, while it is loaded)
     unsigned char *base;
-    int *cells;
+    uint16_t *cells;
     {
         std::lock_guard<std::mutex> lock(g_setup_mutex);
         if (!g_scratch_addr[dev]) {
@@ -187,7 +187,7 @@ extern "C" int wvlh_locham_noalloc(int precision, const int n[3], const int peri
             g_cells_addr[dev] = t;
             g_scratch_addr[dev] = a;
         }
-        cells = (int *)g_cells_addr[dev];
+        cells = (uint16_t *)g_cells_addr[dev];
         base = (unsigned char *)g_scratch_addr[dev];
     }
     cudaStream_t st = (cudaStream_t)stream;

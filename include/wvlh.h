@@ -517,8 +517,8 @@ int wvlh_ks_potential_spin(wvlh_ctx *ctx, int free_bc, const int n[3], const dou
                            const double *rho_dn, const double *rhocore, const double *vext, double *pot_up,
                            double *pot_dn, double *energies);
 /* Measured block size of the plane kernels: times reps calls of
- * wvlh_locham_batched (after one warm-up each) with every block size the
- * kernels are compiled for (FP32 1024/512/384/256/128, FP64 512/384/256/128),
+ * wvlh_locham_batched (after one warm-up each) with the best block
+ * size under each bound the kernels are compiled for (576/384/288/192/128),
  * keeps the fastest in the batch and in a process-wide table keyed by the
  * batch's shape (precision and every orbital's box), which batches of the
  * same shape created later start from.  Arguments as wvlh_locham_batched
