@@ -733,7 +733,10 @@ __device__ __forceinline__ void k2_tile(const LrDev *__restrict__ lrs, const Orb
                     *reinterpret_cast<V *>(B + (z0 + t) * TC + uc) = w;
                 }
             }
-            ep += U::sum(es);
+            // only the plane's own columns count: the pad column of a free row,
+            // which the FP64 K1 leaves as the scratch was, may hold anything,
+            // and 0 * NaN is NaN
+            if (in0) ep += U::n == 1 || in1 ? U::sum(es) : U::first(es);
         }
         e = (double)ep;
         __syncthreads();

@@ -103,6 +103,7 @@ struct U2f {
     static __device__ __forceinline__ V mulv(V c, V x) { return __fmul2_rn(c, x); }
     static __device__ __forceinline__ V zero() { return make_float2(0.f, 0.f); }
     static __device__ __forceinline__ float sum(V a) { return a.x + a.y; }
+    static __device__ __forceinline__ float first(V a) { return a.x; }
     // e += x . r in FP64
     static __device__ __forceinline__ void dot(double &e, V x, V r)
     {
@@ -121,6 +122,7 @@ struct U1d {
     static __device__ __forceinline__ void dot(double &e, V x, V r) { e = ::fma(x, r, e); }
     static __device__ __forceinline__ V zero() { return 0.0; }
     static __device__ __forceinline__ double sum(V a) { return a; }
+    static __device__ __forceinline__ double first(V a) { return a; }
 };
 template <class T> struct ColUnit;
 template <> struct ColUnit<float> { using U = U2f; };

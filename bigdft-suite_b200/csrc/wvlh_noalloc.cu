@@ -279,9 +279,10 @@ extern "C" int wvlh_locham_noalloc(int precision, const int n[3], const int peri
         p.smem_z0[f] = (size_t)(G[2] + I[2]) * TX_ * TY_ * (f ? 8 : 4);
         p.smem_z1[f] = (size_t)G[2] * TX_ * TY_ * (f ? 8 : 4);
     }
-    // the energy slots that are summed, D, Q/Z1 and Z2 are fully
-    // overwritten before they are read, so stale contents of an earlier call
-    // never leak into this one
+    // the energy slots that are summed, D, Z2 and the columns of Q/Z1 are
+    // overwritten before they are read; the pad columns of Q's free rows
+    // travel with their rows, but no result takes them.  So stale contents of
+    // an earlier call never leak into this one
     if (precision == 64)
         e = launch_locham<double, double>(p, (const double *)psi, (const double *)pot, (double *)hpsi,
                                           (double *)(base + o_scr), (double *)(base + o_pp), (double *)(base + o_pk),
