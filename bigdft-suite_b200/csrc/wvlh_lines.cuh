@@ -29,6 +29,12 @@
 // |l| <= 13) and at |l| >= 12 below 6e-11 (FP32 keeps |l| <= 11), against
 // largest taps of 3.6 and 24.9: under a hundredth of one rounding of the sum.
 //
+// FP64 energies: a tap of B off by a rounding moves |B x|^2, and so E_pot and
+// the density, the same way for every orbital.  wvl_composed.h holds the exact
+// sums of products, rounded so that these moves cancel: |B x|^2 is right to 1e-17
+// of itself per axis at every frequency (sums rounded at each step: 4e-16; the
+// nearest doubles: 9e-17), the outputs to 2e-16.
+//
 // FP32 energies: a tap c rounded to FP32 is off by lo = c - fl(c), the same way
 // for every output, and E_kin = <x | T x> by lo(l) sum_i x(i) x(i+l).  The FP32
 // taps of T are kept times kTNorm (the scale -1/(2 h^2) divides by it), a factor
@@ -39,34 +45,18 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include "wvl_composed.h"
 #include "wvlh_common.cuh"
 
 namespace wvlh {
 
 // ---------------------------------------------------------------- taps
-struct BTaps {
-    double s[31], w[31];   // gs(m), gw(m) at m + 14
-    __host__ __device__ constexpr BTaps() : s(), w()
-    {
-        for (int m = -14; m <= 16; ++m) {
-            double a = 0.0, b = 0.0;
-            for (int l = -8; l <= 7; ++l) {
-                const int k = m + l + 7;
-                if (k < 0 || k > 15) continue;
-                a += WVL_MF_AT(l + 8) * WVL_CH_AT(k);
-                b += WVL_MF_AT(l + 8) * WVL_CG_AT(k);
-            }
-            s[m + 14] = a;
-            w[m + 14] = b;
-        }
-    }
-};
-
-// half 0: scaling function, 1: wavelet
+// taps of B: gs (half 0, scaling function) and gw (half 1, wavelet) at m
 __device__ __forceinline__ constexpr double b_tap(int half, int m)
 {
-    constexpr BTaps t{};
-    return m < -14 || m > 16 ? 0.0 : half ? t.w[m + 14] : t.s[m + 14];
+    constexpr double s[31] = WVL_B64_S_INIT;
+    constexpr double w[31] = WVL_B64_W_INIT;
+    return m < -14 || m > 16 ? 0.0 : half ? w[m + 14] : s[m + 14];
 }
 // tap of output half `o` from input half `i` at offset l
 __device__ __forceinline__ constexpr double t_tap(int o, int i, int l)

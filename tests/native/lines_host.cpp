@@ -54,9 +54,7 @@ template <class T> struct Buf {
     }
 };
 
-constexpr int SEG = 8;
-
-template <class T> static void rows(int op, int N, int per, int nrows, const double *in, double *out, double *energy)
+template <class T, int SEG> static void rows(int op, int N, int per, int nrows, const double *in, double *out, double *energy)
 {
     const int H = half_off(N), I = isf_len(N, per), F = fine_len(N, per);
     const int pitch = vec_pitch(max(2 * H, max(F, I)));
@@ -75,7 +73,7 @@ template <class T> static void rows(int op, int N, int per, int nrows, const dou
     *energy = e;
 }
 
-template <class T> static void cols(int op, int N, int per, int ncol, const double *in, double *out, double *energy)
+template <class T, int SEG> static void cols(int op, int N, int per, int ncol, const double *in, double *out, double *energy)
 {
     using U = typename ColUnit<T>::U;
     using V = typename U::V;
@@ -125,12 +123,21 @@ template <class T> static void cols(int op, int N, int per, int ncol, const doub
 }
 
 // op 0: B, 1: B^T, 2: T (rows: 0.25 x - 0.5 T x and <x | -0.5 T x>; columns:
-// T x and <x | T x>); lines are dense rows of in / out
-extern "C" int line_pass(int prec, int as_rows, int op, int N, int per, int nline, const double *in, double *out,
+// T x and <x | T x>); lines are dense rows of in / out; seg: wavelet points of
+// a segment, 6 (FP32 plane kernels, density) or 8
+template <int SEG>
+static void run(int prec, int as_rows, int op, int N, int per, int nline, const double *in, double *out, double *energy)
+{
+    if (as_rows && prec == 32) rows<float, SEG>(op, N, per, nline, in, out, energy);
+    else if (as_rows) rows<double, SEG>(op, N, per, nline, in, out, energy);
+    else if (prec == 32) cols<float, SEG>(op, N, per, nline, in, out, energy);
+    else cols<double, SEG>(op, N, per, nline, in, out, energy);
+}
+extern "C" int line_pass(int prec, int as_rows, int op, int seg, int N, int per, int nline, const double *in, double *out,
                          double *energy)
 {
     g_broken = 0;
-    if (as_rows) prec == 32 ? rows<float>(op, N, per, nline, in, out, energy) : rows<double>(op, N, per, nline, in, out, energy);
-    else prec == 32 ? cols<float>(op, N, per, nline, in, out, energy) : cols<double>(op, N, per, nline, in, out, energy);
+    seg == 6 ? run<6>(prec, as_rows, op, N, per, nline, in, out, energy)
+             : run<8>(prec, as_rows, op, N, per, nline, in, out, energy);
     return g_broken;
 }

@@ -1,12 +1,13 @@
 """The composed line passes of the fused kernels (csrc/wvlh_lines.cuh), built
 for the host: B = magic filter x synthesis, B^T and T = analysis x kinetic x
 synthesis on rows and columns, periodic and free lines, against dense matrices
-made from the filters.  Lengths run from the shortest lines (shorter than the
+made from the filters, in the segment lengths that the kernels use.  Lengths run from the shortest lines (shorter than the
 windows, which wrap several times) over odd ones to several segments with every
 remainder."""
 import ctypes as C
 import re
 import subprocess
+from fractions import Fraction
 from pathlib import Path
 
 import numpy as np
@@ -26,11 +27,11 @@ def line_pass(tmp_path_factory):
                     str(CSRC), str(HERE / "native" / "lines_host.cpp"), "-o", str(so)], check=True)
     f = C.CDLL(str(so)).line_pass
 
-    def call(prec, rows, op, n, per, x, nout):
+    def call(prec, rows, op, n, per, x, nout, seg=8):
         x = np.ascontiguousarray(x)
         out, e = np.zeros((len(x), nout)), C.c_double()
         p = C.POINTER(C.c_double)
-        rc = f(prec, rows, op, n, per, len(x), x.ctypes.data_as(p), out.ctypes.data_as(p), C.byref(e))
+        rc = f(prec, rows, op, seg, n, per, len(x), x.ctypes.data_as(p), out.ctypes.data_as(p), C.byref(e))
         assert rc == 0, "a write outside the buffers"
         return out, e.value
     return call
@@ -65,9 +66,10 @@ def matrices(n, per):
 
 @pytest.mark.parametrize("prec", [64, 32])
 @pytest.mark.parametrize("rows", [1, 0])
+@pytest.mark.parametrize("seg", [6, 8])
 @pytest.mark.parametrize("per,n", [(1, v) for v in (8, 9, 11, 12, 13, 17, 24, 30, 35, 48)] +
                          [(0, v) for v in (1, 2, 3, 5, 6, 7, 12, 13, 18, 31)])
-def test_line_passes_match_dense(line_pass, prec, rows, per, n):
+def test_line_passes_match_dense(line_pass, prec, rows, seg, per, n):
     B, T = matrices(n, per)
     rng = np.random.default_rng(100 * n + per)
     nl = 5
@@ -79,19 +81,21 @@ def test_line_passes_match_dense(line_pass, prec, rows, per, n):
     # partial sum is rounded, so the error is below K eps sum |c|; K <= 62
     eps = 2.0 ** -53 if prec == 64 else 2.0 ** -24
     bound = lambda m: 62 * eps * np.abs(m).sum(axis=1).max()  # noqa: E731
-    got, _ = line_pass(prec, rows, 0, n, per, w, len(B))
+    got, _ = line_pass(prec, rows, 0, n, per, w, len(B), seg)
     assert np.abs(got - w @ B.T).max() <= bound(B)
-    got, _ = line_pass(prec, rows, 1, n, per, r, 2 * n)
+    got, _ = line_pass(prec, rows, 1, n, per, r, 2 * n, seg)
     assert np.abs(got - r @ B).max() <= bound(B.T)
-    got, e = line_pass(prec, rows, 2, n, per, w, 2 * n)
+    got, e = line_pass(prec, rows, 2, n, per, w, 2 * n, seg)
     want = w @ T.T
     ew = (w * want).sum()
     if rows:
         want, ew = 0.25 * w - 0.5 * want, -0.5 * ew
     assert np.abs(got - want).max() <= 2 * bound(T)
-    # the energy of a line: the outputs' errors plus a rounding per term (the
-    # terms of a segment are summed in T)
-    assert abs(e - ew) <= 2 * nl * 2 * n * bound(T)
+    # the energy is x times the outputs: the errors of its up to 62 + 2 seg
+    # roundings a term add up like those of independent steps (six deviations);
+    # the taps' own rounding goes one way, below 3.3e-8 |x|^2 in FP32
+    dev = eps * np.sqrt(62 + 2 * seg) * np.sqrt(((w * (np.abs(w) @ np.abs(T).T)) ** 2).sum())
+    assert abs(e - ew) <= 6 * dev + (3.3e-8 if prec == 32 else 1e-16) * (w * w).sum()
 
 
 def test_fp32_energy_is_not_biased_by_tap_rounding(line_pass):
@@ -105,3 +109,43 @@ def test_fp32_energy_is_not_biased_by_tap_rounding(line_pass):
     for rows in (1, 0):
         _, e = line_pass(32, rows, 2, n, 1, w, 2 * n)
         assert abs(e / (-0.5 if rows else 1.0) - ew) <= 5e-9 * abs(ew)
+
+
+def b_taps(line_pass, prec):
+    """gs(-14..16), gw(-14..16) as the pass holds them: its answers to unit lines"""
+    n = 20
+    x = np.zeros((2, 2 * n))
+    x[0, 3] = x[1, n + 3] = 1.0
+    got, _ = line_pass(prec, 1, 0, n, 0, x, 2 * n + 29)
+    return [Fraction(v) for v in got[:, 6:37].ravel()]     # j = m + 6 is stored at j + 14
+
+
+def tap_bias(taps):
+    """How far the taps' errors D move |B x|^2: the largest eigenvalue over all
+    frequencies of B^T D + D^T B in 2 x 2 symbols (output parity, input half), the
+    largest and the zero-frequency scaling-scaling entry of smooth lines, the
+    mean (white noise); and the largest |D|"""
+    fr = lambda name: [Fraction(v) for v in table(name)]  # noqa: E731
+    mf = fr("MF")
+    exact = [sum((mf[l + 8] * f[m + l + 7] for l in range(-8, 8) if 0 <= m + l + 7 <= 15), Fraction(0))
+             for f in (fr("CH"), fr("CG")) for m in range(-14, 17)]
+    th = np.linspace(0, np.pi, 181)
+    sym = np.zeros((2, len(th), 2, 2), complex)
+    for i, (t, c) in enumerate(zip(taps, exact)):
+        m = i % 31 - 14
+        ph = np.exp(-1j * th * ((m - (m & 1)) // 2))
+        for k, v in enumerate((c, t - c)):
+            sym[k, :, m & 1, i // 31] += float(v) * ph
+    g, d = sym
+    h = np.einsum("toa,tob->tab", g.conj(), d)
+    h = h + np.conj(np.swapaxes(h, 1, 2))
+    ss = np.abs(h[:, 0, 0])
+    return (np.abs(np.linalg.eigvalsh(h)).max(), ss[th < 1].max(), ss[0],
+            abs(np.trace(h, axis1=1, axis2=2).real.mean() / 2), np.linalg.norm(d, 2, axis=(1, 2)).max())
+
+
+def test_fp64_taps_do_not_bias_the_density(line_pass):
+    """|B x|^2 per axis stays within 1e-17 of itself (sums of products rounded
+    at each step: 4e-16, always the same way), the outputs within 2e-16"""
+    worst, smooth, dc, white, dist = tap_bias(b_taps(line_pass, 64))
+    assert worst < 1e-17 and white < 3e-18 and dist < 2e-16
