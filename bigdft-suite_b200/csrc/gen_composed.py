@@ -12,9 +12,17 @@ other, the largest first, each to the neighbour of what the least-squares
 solution for the taps still free asks of it: the least norm of
 B^T D + D^T B over all frequencies, plus LAMBDA |D|^2, which keeps D small.
 
+FP32 taps are kept times NORM, whose -6th power the kernels multiply back (the
+potential's term, E_pot and the density hold six B each): found by a scan of
+[2^-1/2, 2^1/2] in steps of 1e-10 among the factors whose taps lie nearest to
+FP32 values and whose -6th power lies within 2e-9 of one.  Its four largest taps
+take their nearest values, and a local search over the next thirty (steps of a
+few roundings, seeded) balances what measure() returns.
+
 Run ``python gen_composed.py`` to rewrite the header; it is committed, so that the
 build needs neither this script nor numpy.
 """
+import random
 import re
 from fractions import Fraction
 from pathlib import Path
@@ -22,7 +30,10 @@ from pathlib import Path
 import numpy as np
 
 HERE = Path(__file__).resolve().parent
-LAMBDA = 0.01
+NORM = {64: 1.0, 32: 0.9752083272817533}
+BITS = {64: 53, 32: 24}
+LAMBDA = {64: 0.01, 32: 0.1}
+KEEP = {64: 0, 32: 4}
 TH = np.linspace(0.0, np.pi, 129)
 
 
@@ -59,27 +70,62 @@ def rounded(x, bits):
     return round(x / q) * q
 
 
-def least_squares(bits):
+def error(tap, i, prec):
+    return float(tap / Fraction(NORM[prec]) - EXACT[i])
+
+
+def measure(d):
+    """of B^T D + D^T B: the largest eigenvalue, the largest and the
+    zero-frequency scaling-scaling entry (smooth lines), the mean (white noise);
+    and the largest |D|"""
+    M, D = np.tensordot(d, HERM, 1), np.tensordot(d, E, 1)
+    a, b = M[:, 0, 0].real, M[:, 1, 1].real
+    return np.array([np.abs(np.linalg.eigvalsh(M)).max(), np.abs(a[TH < 1]).max(), abs(a[0]), abs((a + b).mean() / 2),
+                     np.linalg.norm(D, 2, axis=(1, 2)).max()])
+
+
+ORDER = sorted(range(62), key=lambda i: -abs(EXACT[i]))
+
+
+def least_squares(prec):
     A = np.stack([HERM[:, :, 0, 0].real, HERM[:, :, 1, 1].real, np.sqrt(2) * HERM[:, :, 0, 1].real,
                   np.sqrt(2) * HERM[:, :, 0, 1].imag], 2).reshape(62, -1).T / np.sqrt(len(TH))
-    A = np.vstack([A, np.sqrt(LAMBDA) * np.eye(62)])
-    free = sorted(range(62), key=lambda i: -abs(EXACT[i]))
+    A = np.vstack([A, np.sqrt(LAMBDA[prec]) * np.eye(62)])
     taps, d = [None] * 62, np.zeros(62)
-    while free:
-        want = np.linalg.lstsq(A[:, free], -A @ d, rcond=None)[0][0]
-        i = free.pop(0)
-        taps[i] = rounded(EXACT[i] + Fraction(want), bits)
-        d[i] = float(taps[i] - EXACT[i])
+    for k, i in enumerate(ORDER):
+        want = 0.0 if k < KEEP[prec] else np.linalg.lstsq(A[:, ORDER[k:]], -A @ d, rcond=None)[0][0]
+        taps[i] = rounded(Fraction(NORM[prec]) * (EXACT[i] + Fraction(want)), BITS[prec])
+        d[i] = error(taps[i], i, prec)
+    return taps
+
+
+def refine(taps, prec):
+    goal = np.array([2.4e-9, 1.2e-9, 6e-10, 3e-10, 8e-9])
+    cost = lambda t: ((measure(np.array([error(v, i, prec) for i, v in enumerate(t)])) / goal) ** 4).sum()  # noqa: E731
+    rng, best, idle = random.Random(1), cost(taps), 0
+    while idle < 3000:
+        t = list(taps)
+        for i in rng.sample(ORDER[4:34], rng.choice((1, 1, 2, 2, 3))):
+            ulp = Fraction(2) ** (int(np.floor(np.log2(abs(float(t[i]))))) + 1 - BITS[prec])
+            t[i] += rng.choice((-1, 1)) * (1 if ulp > 2e-9 else rng.choice((1, 1, 2, 4, 8))) * ulp
+        c = cost(t)
+        taps, best, idle = (t, c, 0) if c < best else (taps, best, idle + 1)
     return taps
 
 
 def render():
     out = ["/* Generated by gen_composed.py from wvl_filters.h; do not edit. */", "#pragma once", ""]
-    taps = least_squares(53)
-    for k, half in enumerate("SW"):
-        out += ["/* taps g%s(-14..16) of magic filter . synthesis (index m+14) */" % half.lower(),
-                "#define WVL_B64_%s_INIT { \\" % half,
-                ", \\\n".join("    %s" % float(t).hex() for t in taps[31 * k:31 * k + 31]) + "}"]
+    for prec in (64, 32):
+        taps = least_squares(prec)
+        if prec == 32:
+            taps = refine(taps, prec)
+        print("FP%d" % prec, *("%.1e" % v for v in measure(np.array([error(t, i, prec) for i, t in enumerate(taps)]))))
+        for k, half in enumerate("SW"):
+            out += ["/* FP%d taps g%s(-14..16) of magic filter . synthesis%s (index m+14) */"
+                    % (prec, half.lower(), ", times %r" % NORM[prec] if NORM[prec] != 1 else ""),
+                    "#define WVL_B%d_%s_INIT { \\" % (prec, half),
+                    ", \\\n".join("    %s%s" % (float(t).hex(), "f" * (prec == 32)) for t in taps[31 * k:31 * k + 31]) + "}"]
+    out += ["/* that factor's -6th power */", "#define WVL_B32_INV6 %s" % float(Fraction(NORM[32]) ** -6).hex()]
     return "\n".join(out) + "\n"
 
 

@@ -1,7 +1,7 @@
 /* Generated by gen_composed.py from wvl_filters.h; do not edit. */
 #pragma once
 
-/* taps gs(-14..16) of magic filter . synthesis (index m+14) */
+/* FP64 taps gs(-14..16) of magic filter . synthesis (index m+14) */
 #define WVL_B64_S_INIT { \
     -0x1.3cf8170a61665p-27, \
     0x1.7584b6cc19e93p-23, \
@@ -34,7 +34,7 @@
     0x1.50f93b4d1f949p-23, \
     -0x1.a76bd1c38b185p-26, \
     0x1.b61f026a675b6p-30}
-/* taps gw(-14..16) of magic filter . synthesis (index m+14) */
+/* FP64 taps gw(-14..16) of magic filter . synthesis (index m+14) */
 #define WVL_B64_W_INIT { \
     -0x1.6237bd7ff8f51p-28, \
     0x1.a16995d0003bap-24, \
@@ -67,3 +67,71 @@
     -0x1.2911ba5f482c4p-22, \
     0x1.7ae531030df92p-25, \
     -0x1.880ca76eac140p-29}
+/* FP32 taps gs(-14..16) of magic filter . synthesis, times 0.9752083272817533 (index m+14) */
+#define WVL_B32_S_INIT { \
+    -0x1.35067c0000000p-27f, \
+    0x1.6c406a0000000p-23f, \
+    -0x1.97ce9c0000000p-20f, \
+    0x1.3f01c80000000p-17f, \
+    -0x1.d1f9f80000000p-16f, \
+    -0x1.1779360000000p-15f, \
+    0x1.17d5980000000p-11f, \
+    -0x1.b98a080000000p-9f, \
+    -0x1.14bc540000000p-8f, \
+    0x1.fca9080000000p-6f, \
+    0x1.76462a0000000p-6f, \
+    -0x1.14aa560000000p-3f, \
+    -0x1.b84f160000000p-4f, \
+    0x1.9f7d700000000p-2f, \
+    0x1.85b06a0000000p-1f, \
+    0x1.a965b40000000p-2f, \
+    -0x1.d7247a0000000p-7f, \
+    -0x1.f44fc60000000p-6f, \
+    0x1.5ddc5e0000000p-5f, \
+    0x1.0050000000000p-7f, \
+    -0x1.ab28960000000p-7f, \
+    -0x1.b60d2c0000000p-10f, \
+    0x1.8d78660000000p-10f, \
+    0x1.ea96e20000000p-13f, \
+    0x1.99f7aa0000000p-16f, \
+    -0x1.cef1980000000p-17f, \
+    0x1.0fabf60000000p-19f, \
+    -0x1.a332ea0000000p-22f, \
+    0x1.48a0880000000p-23f, \
+    -0x1.9cc9080000000p-26f, \
+    0x1.ab8dae0000000p-30f}
+/* FP32 taps gw(-14..16) of magic filter . synthesis, times 0.9752083272817533 (index m+14) */
+#define WVL_B32_W_INIT { \
+    -0x1.58f1340000000p-28f, \
+    0x1.9715a80000000p-24f, \
+    -0x1.cbabc40000000p-21f, \
+    0x1.6dc6940000000p-18f, \
+    -0x1.18eba60000000p-16f, \
+    -0x1.751e0c0000000p-17f, \
+    0x1.2339cc0000000p-12f, \
+    -0x1.f79b5a0000000p-10f, \
+    -0x1.f51e6a0000000p-10f, \
+    0x1.e856c40000000p-7f, \
+    0x1.d1d6b80000000p-8f, \
+    -0x1.3eeae20000000p-5f, \
+    -0x1.a6e6380000000p-5f, \
+    0x1.896fc60000000p-5f, \
+    0x1.92e8620000000p-2f, \
+    -0x1.8602c20000000p-1f, \
+    0x1.b57f620000000p-2f, \
+    0x1.3700280000000p-4f, \
+    -0x1.dd5d320000000p-4f, \
+    -0x1.6d373a0000000p-6f, \
+    0x1.c2ad4e0000000p-6f, \
+    0x1.de86400000000p-9f, \
+    -0x1.5bd8d20000000p-9f, \
+    -0x1.dafe0c0000000p-12f, \
+    -0x1.4cb10e0000000p-15f, \
+    0x1.90a3320000000p-16f, \
+    -0x1.b25f9e0000000p-19f, \
+    0x1.556bd80000000p-21f, \
+    -0x1.21b4a20000000p-22f, \
+    0x1.718bfe0000000p-25f, \
+    -0x1.7f4b980000000p-29f}
+/* that factor's -6th power */
+#define WVL_B32_INV6 0x1.299d91ffff928p+0

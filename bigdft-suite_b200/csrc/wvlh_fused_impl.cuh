@@ -272,13 +272,16 @@ __device__ __forceinline__ void store_wavelet(const T *A, int pitch, const Dims 
                   [&](int so, int go) { *reinterpret_cast<V *>(g + go) = *reinterpret_cast<const V *>(A + so); });
 }
 
-// A += the dense wavelet plane g
+// A = scale A + the dense wavelet plane g
 template <class T>
-__device__ __forceinline__ void add_wavelet(T *A, int pitch, const Dims &d, const T *__restrict__ g)
+__device__ __forceinline__ void scale_add_wavelet(T *A, int pitch, const Dims &d, T scale, const T *__restrict__ g)
 {
     if (d.N1 & 1) {
         RowCol q(d.G1);
-        for (int i = threadIdx.x; i < d.G2 * d.G1; i += blockDim.x, q.next()) A[q.r * pitch + wcol(d, q.c)] += g[i];
+        for (int i = threadIdx.x; i < d.G2 * d.G1; i += blockDim.x, q.next()) {
+            T *a = A + q.r * pitch + wcol(d, q.c);
+            *a = fma(scale, *a, g[i]);
+        }
         return;
     }
     using V = typename Pair<T>::type;
@@ -286,8 +289,8 @@ __device__ __forceinline__ void add_wavelet(T *A, int pitch, const Dims &d, cons
         const V v = *reinterpret_cast<const V *>(g + go);
         V *a = reinterpret_cast<V *>(A + so);
         V r = *a;
-        r.x += v.x;
-        r.y += v.y;
+        r.x = fma(scale, r.x, v.x);
+        r.y = fma(scale, r.y, v.y);
         *a = r;
     });
 }
@@ -738,7 +741,7 @@ __device__ __forceinline__ void k2_tile(const LrDev *__restrict__ lrs, const Orb
             // and 0 * NaN is NaN
             if (in0) ep += U::n == 1 || in1 ? U::sum(es) : U::first(es);
         }
-        e = (double)ep;
+        e = (double)ep * BInv6<T>::v;
         __syncthreads();
         for (int s = sg; s * kSegZ < d.N3; s += DS) {
             const int i0 = s * kSegZ;
@@ -866,7 +869,7 @@ __device__ __forceinline__ void k3_item(const LrDev *__restrict__ lrs, const Orb
         // 24 x 48^3, where that pass computes for 26)
         const T *z2 = scratch + o.sZ + wofs;
         if (MODE == MODE_PRECOND) load_wavelet<T, true>(A, pitch, d, z2);
-        else add_wavelet(A, pitch, d, z2);
+        else scale_add_wavelet(A, pitch, d, (T)BInv6<T>::v, z2);
         cp_async_wait_all();
         __syncthreads();
         // e: the kinetic energy partial (MODE_LOCHAM) or <d | A d>
@@ -1023,7 +1026,7 @@ __global__ void __launch_bounds__(kZThreads, MAXP > 32 ? 1 : 2) kd_density(const
                 if (2 * s * kDenSeg + t < d.I3) *reinterpret_cast<typename U::V *>(B + (2 * s * kDenSeg + t) * TC + uc) = r[t];
         }
         __syncthreads();
-        const double hf = hfac[orb];
+        const double hf = hfac[orb] * BInv6<T>::v;
 #pragma unroll
         for (int k = 0; k < MAXP; ++k) {
             const int i = threadIdx.x + k * blockDim.x;

@@ -41,7 +41,12 @@
 // found by search so that all the large taps round to within 7e-9 of
 // themselves (unscaled: e(0) by 8e-7, a(1), e(1) by 1e-7): under 4e-8 Ha per
 // axis on a normalised orbital at h = 0.45, with nothing to compute for it.
-// B's residuals move |r|^2 by 2e-9 of itself per axis, below the rounding of r.
+// B's FP32 taps are kept times 0.9752 and rounded as in FP64: |B x|^2 is
+// right to 2.1e-9 of itself per axis at every frequency and to 6e-10 on smooth
+// lines (nearest FP32 taps: 3.1e-8 and 2.4e-8, all smooth orbitals the same way),
+// the outputs to 1.1e-8 (2.3e-8).  E_pot, the potential's term of H psi and the
+// density each hold six B: BInv6 comes in where they are formed (once a thread,
+// in K3's addition of Z2, on the orbital's factor), at no cost.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -51,13 +56,21 @@
 namespace wvlh {
 
 // ---------------------------------------------------------------- taps
-// taps of B: gs (half 0, scaling function) and gw (half 1, wavelet) at m
-__device__ __forceinline__ constexpr double b_tap(int half, int m)
+// taps of B (FP32: times 0.9752, gen_composed.py): gs (half 0, scaling function) and gw
+// (half 1, wavelet) at m
+template <class T> __device__ __forceinline__ constexpr T b_tap(int half, int m)
 {
-    constexpr double s[31] = WVL_B64_S_INIT;
-    constexpr double w[31] = WVL_B64_W_INIT;
-    return m < -14 || m > 16 ? 0.0 : half ? w[m + 14] : s[m + 14];
+    if (m < -14 || m > 16) return T(0);
+    if constexpr (sizeof(T) == 4) {
+        constexpr T s[31] = WVL_B32_S_INIT, w[31] = WVL_B32_W_INIT;
+        return half ? w[m + 14] : s[m + 14];
+    } else {
+        constexpr T s[31] = WVL_B64_S_INIT, w[31] = WVL_B64_W_INIT;
+        return half ? w[m + 14] : s[m + 14];
+    }
 }
+// what six passes of scaled taps (B on three axes, twice) are multiplied by
+template <class T> struct BInv6 { static constexpr double v = sizeof(T) == 4 ? WVL_B32_INV6 : 1.0; };
 // tap of output half `o` from input half `i` at offset l
 __device__ __forceinline__ constexpr double t_tap(int o, int i, int l)
 {
@@ -226,7 +239,7 @@ __device__ __forceinline__ void b_point(typename U::V (&acc)[2 * HS], int k, typ
 #pragma unroll
         for (int o = 0; o < 2; ++o) {
             const int m = 16 + o - 2 * (k - t);
-            if (m >= -14 && m <= 16) acc[2 * t + o] = U::fma((typename U::T)b_tap(half, m), x, acc[2 * t + o]);
+            if (m >= -14 && m <= 16) acc[2 * t + o] = U::fma(b_tap<typename U::T>(half, m), x, acc[2 * t + o]);
         }
 }
 // c[t], d[t] (coarse point i0 + t of B^T) from x = r(2 i0 - 14 + k)
@@ -238,8 +251,8 @@ __device__ __forceinline__ void bt_point(typename U::V (&c)[HS], typename U::V (
     for (int t = 0; t < HS; ++t) {
         const int m = k - 14 - 2 * t;
         if (m < -14 || m > 16) continue;
-        c[t] = U::fma((T)b_tap(0, m), x, c[t]);
-        d[t] = U::fma((T)b_tap(1, m), x, d[t]);
+        c[t] = U::fma(b_tap<T>(0, m), x, c[t]);
+        d[t] = U::fma(b_tap<T>(1, m), x, d[t]);
     }
 }
 // s[t], w[t] (coarse point i0 + t of TNorm T) from x = point i0 - R + k of input half i

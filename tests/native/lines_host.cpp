@@ -122,7 +122,9 @@ template <class T, int SEG> static void cols(int op, int N, int per, int ncol, c
     *energy = e;
 }
 
-// op 0: B, 1: B^T, 2: T (rows: 0.25 x - 0.5 T x and <x | -0.5 T x>; columns:
+extern "C" double b_inv6(int prec) { return prec == 32 ? BInv6<float>::v : BInv6<double>::v; }
+
+// op 0: B, 1: B^T (FP32: scaled as the taps are), 2: T (rows: 0.25 x - 0.5 T x and <x | -0.5 T x>; columns:
 // T x and <x | T x>); lines are dense rows of in / out; seg: wavelet points of
 // a segment, 6 (FP32 plane kernels, density) or 8
 template <int SEG>
