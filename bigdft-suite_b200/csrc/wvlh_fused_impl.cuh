@@ -664,13 +664,18 @@ __device__ __forceinline__ void k2_tile(const LrDev *__restrict__ lrs, const Orb
         }
         const bool ok = mbar_wait_bounded(tma_bar, 0);
         if (!__syncthreads_and(ok)) {
-            // the copy did not complete in time: poison this tile's energy
-            // slot (the orbital's energies come out NaN), give the copy in
-            // flight one more bounded wait and leave the tile
+            // the copy did not complete in time: give it one more bounded wait,
+            // then leave NaN in place of the tile's results (what the orbital's
+            // Hpsi or CG vectors take) and in its energy slot
             if (threadIdx.x == 0) {
-                if (part_kin)
-                    (chain == 0 ? part_pot : part_kin)[(size_t)oi * part_stride + jj] = __longlong_as_double(-1LL);
                 mbar_wait_bounded(tma_bar, 0);
+                if (EN && part_kin)
+                    (chain == 0 ? part_pot : part_kin)[(size_t)oi * part_stride + jj] = __longlong_as_double(-1LL);
+            }
+            __syncthreads();
+            for (int i = threadIdx.x; i < TC * d.G3; i += blockDim.x) {
+                const int c = i % TC, x = x0 + c % TX, y = y0 + c / TX;
+                if (x < W && y < H) gz[(i / TC) * plane + (size_t)y * WP + x] = (T)__longlong_as_double(-1LL);
             }
             return;
         }

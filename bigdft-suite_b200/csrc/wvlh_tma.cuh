@@ -10,7 +10,8 @@
 // (the source is this GPU's own memory).
 //
 // Every wait on the mbarrier is bounded: after kTmaSpinLimit polls the CTA
-// records an error in the batch's flag and returns without using the tile.
+// waits once more as long, writes NaN for the tile's results and energy, and
+// returns without using the tile.
 #pragma once
 #include <cuda.h>
 #include <cuda_runtime.h>
