@@ -353,7 +353,7 @@ static void layout(wvlh_batch *b, const std::vector<int> &orb_lr, const std::vec
         q.sP = scr;
         q.sZ = scr + sc.z;
         q.sQ = scr + sc.q;
-        scr += (sc.total + 3) & ~3LL;   // orbitals start on 16 bytes (TMA strides)
+        scr += sc.stride();
         q.c = 0.0;
         q.in_ptr = abs ? abs[o].psi : nullptr;
         q.out_ptr = abs ? abs[o].hpsi : nullptr;
@@ -395,7 +395,7 @@ static void layout(wvlh_batch *b, const std::vector<int> &orb_lr, const std::vec
     p.psi_total = psi_off;
     p.all_periodic = true;
     for (int v : p.lr_per) p.all_periodic = p.all_periodic && v == 1;
-    p.scratch_elems = (scr + 1) & ~1LL;  // even: the global plane slices after it start on a point pair
+    p.scratch_elems = scr;  // even: the global plane slices after it start on a point pair
     {
         // one region for every orbital: regular (x, y, z, orbital) plane tensors
         bool one = norb > 0;
@@ -403,7 +403,7 @@ static void layout(wvlh_batch *b, const std::vector<int> &orb_lr, const std::vec
         if (one) {
             const LrDev &d = lrd[orb_lr[0]];
             const OrbScratch sc = orb_scratch(d.N, d.per);
-            p.orb_scratch = (sc.total + 3) & ~3LL;
+            p.orb_scratch = sc.stride();
             p.tile = TileDims{2LL * d.N[0], 2LL * d.N[1], 2LL * d.N[2], isf_len(d.N[0], d.per[0]),
                               isf_pitch(d.N[0], d.per[0]), isf_len(d.N[1], d.per[1]), sc.q};
         }

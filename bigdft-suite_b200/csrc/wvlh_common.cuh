@@ -55,6 +55,9 @@ __host__ __device__ __forceinline__ int isf_pitch(int N, int per) { return per ?
 // covers Q's padded rows.
 struct OrbScratch {
     long long z, q, total;
+    // from one orbital of a batch to the next: on 16 bytes of FP32 (TMA strides),
+    // and never more than callers budget; Q's last row ends well before
+    __host__ __device__ long long stride() const { return total & ~3LL; }
 };
 __host__ __device__ inline OrbScratch orb_scratch(const int *N, const int *per)
 {

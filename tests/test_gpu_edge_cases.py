@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 
 from wvlh._lib import WvlhError
-from wvlh.batch import Batch
+from wvlh.batch import Batch, Region
 from wvlh.keys import Locreg
 
 pytestmark = pytest.mark.gpu
@@ -145,3 +145,14 @@ def test_mixed_boundary_conditions_in_one_batch(oracle, torch_cuda, wctx):
         assert rel(h[b.psi_offset(o):b.psi_offset(o) + lrs[r].ncoeff], ref) < 1e-13
         assert abs(ek[o] - e1) <= 1e-12 * abs(e1) and abs(ep[o] - e2) <= 1e-12 * abs(e2)
     b.close()
+
+
+@pytest.mark.parametrize("N,per", [((8, 7, 9), (0, 0, 0)), ((9, 8, 9), (0, 0, 1)), ((8, 9, 11), (1, 0, 1))])
+@pytest.mark.parametrize("prec", [32, 64])
+def test_batch_scratch_within_its_orbitals(wctx, N, per, prec):
+    """A batch takes no more scratch than its orbitals' wvlh_region_scratch_bytes
+    add up to, which is what a caller budgets by."""
+    lr, _ = region(N, per, 0.5, 11)
+    one = Region(wctx, lr).scratch_bytes(prec)
+    for norb in (1, 2, 5):
+        assert Batch(wctx, [lr], [0] * norb).scratch_bytes(prec) <= norb * one
