@@ -135,3 +135,68 @@
     -0x1.7f4b980000000p-29f}
 /* that factor's -6th power */
 #define WVL_B32_INV6 0x1.299d91ffff928p+0
+/* FP64 taps a(0..14) of analysis . kinetic . synthesis */
+#define WVL_T64_A_INIT { \
+    -0x1.c6df63929cbc6p+1, \
+    0x1.1c0cfedee564dp+1, \
+    -0x1.3b31c704d5a7cp-1, \
+    0x1.e5bd9c1ae926bp-3, \
+    -0x1.50f692972eaedp-4, \
+    0x1.69998376f173bp-6, \
+    -0x1.0c8b4658f56fap-8, \
+    0x1.d99eb6795ef2ep-12, \
+    -0x1.925b217cd373ap-16, \
+    0x1.18926785388d8p-19, \
+    -0x1.8fc3246778128p-22, \
+    -0x1.6bb8d9c92ea58p-27, \
+    -0x1.ff64ebd74464ap-35, \
+    0x1.30e1578b337e4p-42, \
+    0x0.0p+0}
+/* FP64 taps c(-14..14) of analysis . kinetic . synthesis (index l+14) */
+#define WVL_T64_C_INIT { \
+    0x0.0p+0, \
+    0x1.54b5f0ae59996p-43, \
+    -0x1.1bcda68fe9ddap-35, \
+    -0x1.99c0098fe4b7bp-28, \
+    -0x1.d113af7c23d26p-23, \
+    0x1.d848a400104a4p-21, \
+    -0x1.7c5330f6b7d95p-17, \
+    0x1.c74ef21ac362dp-13, \
+    -0x1.17ebd3009653cp-9, \
+    0x1.d3c542e7740dcp-8, \
+    -0x1.d2723a0ac45ffp-6, \
+    0x1.256c77f0a4f52p-3, \
+    -0x1.b32e1735e41f7p-2, \
+    0x1.5066554a2523fp-1, \
+    -0x1.aeea88d1ec73ap-2, \
+    -0x1.bcbeff8673da3p-3, \
+    0x1.44e667bf88ca4p-1, \
+    -0x1.10e30c511a2b7p-1, \
+    0x1.dea0ad8c63400p-3, \
+    -0x1.cf7b581657694p-5, \
+    0x1.09006013021ffp-7, \
+    -0x1.e9cf108a9bb0ap-11, \
+    0x1.a9ca254ac1755p-15, \
+    -0x1.366b75cd07305p-18, \
+    0x1.5729c80321a62p-21, \
+    0x1.42d35b090d4eep-26, \
+    0x1.ccba493c1cf33p-34, \
+    -0x1.10d7b7f7fe198p-41, \
+    0x0.0p+0}
+/* FP64 taps e(0..14) of analysis . kinetic . synthesis */
+#define WVL_T64_E_INIT { \
+    -0x1.8e0377204924fp+4, \
+    -0x1.c9384674485a3p+2, \
+    -0x1.5c4cb92590702p-5, \
+    -0x1.147036d893417p-2, \
+    0x1.502d650670453p-4, \
+    -0x1.69a6019014afbp-6, \
+    0x1.0c8b445990809p-8, \
+    -0x1.d99eb6795f3abp-12, \
+    0x1.925b217cd3652p-16, \
+    -0x1.189267853c2dfp-19, \
+    0x1.8fc3246774392p-22, \
+    0x1.6bb8d9c5727b3p-27, \
+    0x1.ff64eec400352p-35, \
+    -0x1.30e69e4e8bbc9p-42, \
+    0x0.0p+0}

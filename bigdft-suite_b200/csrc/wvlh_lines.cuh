@@ -25,15 +25,20 @@
 // they replace were bound by instruction issue, half of it addressing, window
 // loads and stores.
 //
-// Taps left out of T: |a|, |c|, |e| at |l| = 14 are below 7e-18 (FP64 keeps
-// |l| <= 13) and at |l| >= 12 below 6e-11 (FP32 keeps |l| <= 11), against
-// largest taps of 3.6 and 24.9: under a hundredth of one rounding of the sum.
+// Taps left out of T: at |l| = 14 (FP64 keeps |l| <= 13) they are up to 1.2e-17,
+// 3.0e-17 in all for an output, a seventh of half a rounding of the largest
+// scaling tap, 3.55; at |l| >= 12 (FP32 keeps |l| <= 11) up to 1.05e-10, 2.5e-10
+// in all, 1/470 of half a rounding.
 //
 // FP64 energies: a tap of B off by a rounding moves |B x|^2, and so E_pot and
 // the density, the same way for every orbital.  wvl_composed.h holds the exact
 // sums of products, rounded so that these moves cancel: |B x|^2 is right to 1e-17
 // of itself per axis at every frequency (sums rounded at each step: 4e-16; the
-// nearest doubles: 9e-17), the outputs to 2e-16.
+// nearest doubles: 9e-17), the outputs to 2e-16.  E_kin of a smooth orbital is a
+// small difference of large terms: T's taps are those of the same doubles as
+// the separate passes (not the published a, c, e of the many-digit filters, off
+// by 1e-15 at zero frequency), rounded so that the scaling part is right to 3e-19
+// at zero frequency and 4e-18 below 0.5, the rest to 1e-15 of T's norm of 40.
 //
 // FP32 energies: a tap c rounded to FP32 is off by lo = c - fl(c), the same way
 // for every output, and E_kin = <x | T x> by lo(l) sum_i x(i) x(i+l).  The FP32
@@ -74,9 +79,9 @@ template <class T> struct BInv6 { static constexpr double v = sizeof(T) == 4 ? W
 // tap of output half `o` from input half `i` at offset l
 __device__ __forceinline__ constexpr double t_tap(int o, int i, int l)
 {
-    constexpr double a[15] = WVL_KIN_INIT;
-    constexpr double c[29] = WVL_KIN_C_INIT;
-    constexpr double e[15] = WVL_KIN_E_INIT;
+    constexpr double a[15] = WVL_T64_A_INIT;
+    constexpr double c[29] = WVL_T64_C_INIT;
+    constexpr double e[15] = WVL_T64_E_INIT;
     const int al = l < 0 ? -l : l;
     return al > 14 ? 0.0 : o == i ? (o ? e[al] : a[al]) : (o ? c[l + 14] : c[14 - l]);
 }

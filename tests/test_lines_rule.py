@@ -177,3 +177,35 @@ def test_fp32_norms_of_smooth_and_rough_lines(line_pass):
         for rows in (1, 0):
             got, _ = line_pass(32, rows, 0, n, 1, w, 2 * n)
             assert abs((got ** 2).sum() / want - 1) < 1.5e-9, name
+
+
+def t_symbol_errors(line_pass, prec):
+    """The errors of T's taps (answers to unit lines) against 4 analysis .
+    kinetic . synthesis of the filters' doubles, as 2 x 2 symbols: the scaling-
+    scaling entry at frequency 0 and below 0.5, and the largest norm"""
+    n, mid = 40, 20
+    x = np.zeros((2, 2 * n))
+    x[0, mid] = x[1, n + mid] = 1.0
+    got, _ = line_pass(prec, 0, 2, n, 0, x, 2 * n)
+    kin, fine = [Fraction(v) for v in table("KIN")], [[Fraction(v) for v in table(t)] for t in ("CH", "CG")]
+    th = np.linspace(0, np.pi, 181)
+    d = np.zeros((len(th), 2, 2), complex)
+    for i in range(2):
+        y = {}
+        for p in range(16):
+            for l in range(-14, 15):
+                y[p + l] = y.get(p + l, 0) + kin[abs(l)] * fine[i][p]
+        for o in range(2):
+            for l in range(-14, 15):
+                want = 4 * sum((fine[o][p] * y.get(2 * l + p, 0) for p in range(16)), Fraction(0))
+                d[:, o, i] += float(Fraction(got[i, o * n + mid + l]) - want) * np.exp(-1j * th * l)
+    ss = np.abs(d[:, 0, 0])
+    return ss[0], ss[th < 0.5].max(), np.linalg.norm(d, 2, axis=(1, 2)).max()
+
+
+def test_fp64_taps_do_not_bias_the_kinetic_energy(line_pass):
+    """<x | T x> of smooth orbitals is a small difference of large terms: T's
+    scaling part is right to 1e-18 at frequency 0 (the published tables of a, c,
+    e, taps of the many-digit filters: 1e-15), T's norm is 40"""
+    zero, low, worst = t_symbol_errors(line_pass, 64)
+    assert zero < 1e-18 and low < 1e-17 and worst < 1.2e-15
