@@ -26,7 +26,7 @@ differs by 1e-15 at zero frequency, where a smooth orbital's kinetic energy has
 nothing else).  Their errors D enter E_kin as <x | D x>, so they are
 rounded in turn likewise, the norm of D weighted by 1 / (theta^2 + 0.03) in its
 scaling-scaling part, where orbitals live.  The taps left out (T_REACH) count
-as errors.
+as errors.  FP32 taps are kept times T_NORM, found by a scan like NORM.
 
 Run ``python gen_composed.py`` to rewrite the header; it is committed, so that the
 build needs neither this script nor numpy.
@@ -129,8 +129,8 @@ def refine(taps, prec):
     return taps
 
 
-T_NORM = {64: 1.0}
-T_REACH = {64: 13}
+T_NORM = {64: 1.0, 32: 1.9474363232066856}
+T_REACH = {64: 13, 32: 11}
 T_TAPS = [("A", l) for l in range(15)] + [("C", l) for l in range(-14, 15)] + [("E", l) for l in range(15)]
 
 
@@ -187,12 +187,13 @@ def render():
             out += define("B%d_%s" % (prec, half), "FP%d taps g%s(-14..16) of magic filter . synthesis%s (index m+14)"
                           % (prec, half.lower(), times(NORM[prec])), taps[31 * k:31 * k + 31], prec)
     out += ["/* that factor's -6th power */", "#define WVL_B32_INV6 %s" % float(Fraction(NORM[32]) ** -6).hex()]
-    for prec in (64,):
+    for prec in (64, 32):
         taps = t_taps(prec)
         for k, what in (("A", "a(0..14)"), ("C", "c(-14..14)"), ("E", "e(0..14)")):
             out += define("T%d_%s" % (prec, k), "FP%d taps %s of analysis . kinetic . synthesis%s%s"
                           % (prec, what, times(T_NORM[prec]), " (index l+14)" if k == "C" else ""),
                           [t for t, (q, _) in zip(taps, T_TAPS) if q == k], prec)
+    out += ["/* that factor */", "#define WVL_T32_NORM %r" % T_NORM[32]]
     return "\n".join(out) + "\n"
 
 

@@ -200,3 +200,70 @@
     0x1.ff64eec400352p-35, \
     -0x1.30e69e4e8bbc9p-42, \
     0x0.0p+0}
+/* FP32 taps a(0..14) of analysis . kinetic . synthesis, times 1.9474363232066856 */
+#define WVL_T32_A_INIT { \
+    -0x1.baeaf00000000p+2f, \
+    0x1.1495dc0000000p+2f, \
+    -0x1.32e91a0000000p+0f, \
+    0x1.d8f9780000000p-2f, \
+    -0x1.481b6e0000000p-3f, \
+    0x1.60189e0000000p-5f, \
+    -0x1.057c740000000p-7f, \
+    0x1.cd2bec0000000p-11f, \
+    -0x1.87c76e0000000p-15f, \
+    0x1.1131820000000p-18f, \
+    -0x1.852e040000000p-21f, \
+    -0x1.65f3ea0000000p-26f, \
+    0x0.0p+0f, \
+    0x0.0p+0f, \
+    0x0.0p+0f}
+/* FP32 taps c(-14..14) of analysis . kinetic . synthesis, times 1.9474363232066856 (index l+14) */
+#define WVL_T32_C_INIT { \
+    0x0.0p+0f, \
+    0x0.0p+0f, \
+    0x0.0p+0f, \
+    -0x1.91ab880000000p-27f, \
+    -0x1.c4fc820000000p-22f, \
+    0x1.cbd9aa0000000p-20f, \
+    -0x1.7254d60000000p-16f, \
+    0x1.bb578a0000000p-12f, \
+    -0x1.10907a0000000p-8f, \
+    0x1.c77a080000000p-7f, \
+    -0x1.c62fe80000000p-5f, \
+    0x1.1db6460000000p-2f, \
+    -0x1.a7be220000000p-1f, \
+    0x1.478efc0000000p+0f, \
+    -0x1.a397440000000p-1f, \
+    -0x1.b10eae0000000p-2f, \
+    0x1.3c5c6e0000000p+0f, \
+    -0x1.09b7060000000p+0f, \
+    0x1.d20c660000000p-2f, \
+    -0x1.c34cf80000000p-4f, \
+    0x1.0209680000000p-6f, \
+    -0x1.dcef900000000p-10f, \
+    0x1.9e993c0000000p-14f, \
+    -0x1.2e43940000000p-17f, \
+    0x1.4e1c720000000p-20f, \
+    0x1.39ab400000000p-25f, \
+    0x0.0p+0f, \
+    0x0.0p+0f, \
+    0x0.0p+0f}
+/* FP32 taps e(0..14) of analysis . kinetic . synthesis, times 1.9474363232066856 */
+#define WVL_T32_E_INIT { \
+    -0x1.838d920000000p+5f, \
+    -0x1.bd34080000000p+3f, \
+    -0x1.5325500000000p-4f, \
+    -0x1.0d2c4c0000000p-1f, \
+    0x1.47578a0000000p-3f, \
+    -0x1.6024c80000000p-5f, \
+    0x1.057c760000000p-7f, \
+    -0x1.cd2c220000000p-11f, \
+    0x1.87c85a0000000p-15f, \
+    -0x1.1133400000000p-18f, \
+    0x1.8556d60000000p-21f, \
+    0x1.6195cc0000000p-26f, \
+    0x0.0p+0f, \
+    0x0.0p+0f, \
+    0x0.0p+0f}
+/* that factor */
+#define WVL_T32_NORM 1.9474363232066856

@@ -42,10 +42,12 @@
 //
 // FP32 energies: a tap c rounded to FP32 is off by lo = c - fl(c), the same way
 // for every output, and E_kin = <x | T x> by lo(l) sum_i x(i) x(i+l).  The FP32
-// taps of T are kept times kTNorm (the scale -1/(2 h^2) divides by it), a factor
-// found by search so that all the large taps round to within 7e-9 of
-// themselves (unscaled: e(0) by 8e-7, a(1), e(1) by 1e-7): under 4e-8 Ha per
-// axis on a normalised orbital at h = 0.45, with nothing to compute for it.
+// taps of T are kept times TNorm (the scale -1/(2 h^2) divides by it), a factor
+// found by a scan so that the taps above 0.02 round to within 7.5e-9 (unscaled: up to
+// 8.3e-7), and rounded in turn: the scaling part is right to 2.2e-11 at zero
+// frequency and 1.9e-9 below 0.5 (nearest values: 1.5e-8), all of T to 3.9e-8,
+// times 1 / (2 h^2) in Ha per axis on a normalised orbital (h = 0.45: 5e-11, 5e-9
+// and 1e-7; the separate passes with their corrections: 4e-8, 4e-8 and 3e-7).
 // B's FP32 taps are kept times 0.9752 and rounded as in FP64: |B x|^2 is
 // right to 2.1e-9 of itself per axis at every frequency and to 6e-10 on smooth
 // lines (nearest FP32 taps: 3.1e-8 and 2.4e-8, all smooth orbitals the same way),
@@ -76,17 +78,21 @@ template <class T> __device__ __forceinline__ constexpr T b_tap(int half, int m)
 }
 // what six passes of scaled taps (B on three axes, twice) are multiplied by
 template <class T> struct BInv6 { static constexpr double v = sizeof(T) == 4 ? WVL_B32_INV6 : 1.0; };
-// tap of output half `o` from input half `i` at offset l
-__device__ __forceinline__ constexpr double t_tap(int o, int i, int l)
+// tap of output half `o` from input half `i` at offset l of TNorm T
+template <class V> __device__ __forceinline__ constexpr V t_tap(int o, int i, int l)
 {
-    constexpr double a[15] = WVL_T64_A_INIT;
-    constexpr double c[29] = WVL_T64_C_INIT;
-    constexpr double e[15] = WVL_T64_E_INIT;
     const int al = l < 0 ? -l : l;
-    return al > 14 ? 0.0 : o == i ? (o ? e[al] : a[al]) : (o ? c[l + 14] : c[14 - l]);
+    if (al > 14) return V(0);
+    if constexpr (sizeof(V) == 4) {
+        constexpr V a[15] = WVL_T32_A_INIT, c[29] = WVL_T32_C_INIT, e[15] = WVL_T32_E_INIT;
+        return o == i ? (o ? e[al] : a[al]) : (o ? c[l + 14] : c[14 - l]);
+    } else {
+        constexpr V a[15] = WVL_T64_A_INIT, c[29] = WVL_T64_C_INIT, e[15] = WVL_T64_E_INIT;
+        return o == i ? (o ? e[al] : a[al]) : (o ? c[l + 14] : c[14 - l]);
+    }
 }
 template <class T> struct TReach { static constexpr int v = sizeof(T) == 4 ? 11 : 13; };
-template <class T> struct TNorm { static constexpr double v = sizeof(T) == 4 ? 1.9474363232066856 : 1.0; };
+template <class T> struct TNorm { static constexpr double v = sizeof(T) == 4 ? WVL_T32_NORM : 1.0; };
 
 // ---------------------------------------------------------------- units
 // What one thread carries of a point: a column pass takes 8 bytes of a row of
@@ -269,8 +275,8 @@ __device__ __forceinline__ void t_point(typename U::V (&s)[SEG], typename U::V (
     for (int t = 0; t < SEG; ++t) {
         const int l = k - R - t;
         if (l < -R || l > R) continue;
-        s[t] = U::fma((T)(TNorm<T>::v * t_tap(0, i, l)), x, s[t]);
-        w[t] = U::fma((T)(TNorm<T>::v * t_tap(1, i, l)), x, w[t]);
+        s[t] = U::fma(t_tap<T>(0, i, l), x, s[t]);
+        w[t] = U::fma(t_tap<T>(1, i, l), x, w[t]);
     }
 }
 template <class U, int n>

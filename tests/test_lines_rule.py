@@ -209,3 +209,10 @@ def test_fp64_taps_do_not_bias_the_kinetic_energy(line_pass):
     e, taps of the many-digit filters: 1e-15), T's norm is 40"""
     zero, low, worst = t_symbol_errors(line_pass, 64)
     assert zero < 1e-18 and low < 1e-17 and worst < 1.2e-15
+
+
+def test_fp32_taps_do_not_bias_the_kinetic_energy(line_pass):
+    """The FP32 form: 1e-10 at frequency 0, 3e-9 below 0.5 (nearest values of the
+    scaled taps: 1.5e-8 throughout)"""
+    zero, low, worst = t_symbol_errors(line_pass, 32)
+    assert zero < 1e-10 and low < 3e-9 and worst < 4.2e-8
