@@ -156,3 +156,49 @@ def test_batch_scratch_within_its_orbitals(wctx, N, per, prec):
     one = Region(wctx, lr).scratch_bytes(prec)
     for norb in (1, 2, 5):
         assert Batch(wctx, [lr], [0] * norb).scratch_bytes(prec) <= norb * one
+
+
+@pytest.mark.parametrize("dtype_name,tol", [("float64", 1e-13), ("float32", 1e-6)])
+def test_shared_and_separate_cell_tables_in_one_batch(oracle, torch_cuda, wctx, dtype_name, tol):
+    """Regions whose cells are all fine (one cell table for both key sets), some
+    fine (two) and none, in one batch, odd and even row lengths."""
+    torch, dt = torch_cuda, getattr(torch_cuda, dtype_name)
+    lrs = [region(N, per, dens, 20 + i)[0] for i, (N, per, dens) in enumerate(
+        [((9, 8, 10), (1, 1, 1), 2.0), ((8, 9, 8), (0, 0, 0), 0.4), ((10, 8, 9), (1, 0, 1), 0.0), ((7, 6, 5), (0, 0, 0), 2.0)])]
+    assert lrs[0].nvctr_f == lrs[0].nvctr_c and 0 < lrs[1].nvctr_f < lrs[1].nvctr_c and lrs[2].nvctr_f == 0
+    off = np.cumsum([0] + [lr.nisf for lr in lrs])
+    orb = [1, 0, 2, 3, 0, 1]
+    b = Batch(wctx, lrs, orb, off[orb])
+    rng = np.random.default_rng(6)
+    psi, pot = rng.uniform(-1, 1, b.psi_size), rng.uniform(-1, 0, int(off[-1]))
+    h, ek, ep = b.locham(torch.tensor(psi, dtype=dt, device="cuda"), torch.tensor(pot, dtype=dt, device="cuda"))
+    h = h.double().cpu().numpy()
+    for o, l in enumerate(orb):
+        s = slice(b.psi_offset(o), b.psi_offset(o) + lrs[l].ncoeff)
+        ref, e1, e2 = oracle_locham(oracle, lrs[l], psi[s], pot[off[l]:off[l + 1]])
+        assert rel(h[s], ref) < tol
+        assert abs(ek[o].item() - e1) <= 10 * tol * abs(e1) and abs(ep[o].item() - e2) <= 10 * tol * abs(e2)
+
+
+@pytest.mark.parametrize("dtype_name,etol", [("float64", 1e-14), ("float32", 1e-6)])
+@pytest.mark.parametrize("N,per", [((16, 16, 16), (1, 1, 1)), ((13, 12, 11), (0, 0, 0)), ((17, 9, 24), (1, 0, 0))])
+def test_one_launch_for_both_z_chains_or_two(torch_cuda, wctx, N, per, dtype_name, etol):
+    """The most orbitals whose z tiles of both chains fit two to an SM run them in
+    one launch, one orbital more in two: Hpsi the same bits, the energies the
+    same but for the order of their sums (other numbers of threads a tile)."""
+    torch, dt = torch_cuda, getattr(torch_cuda, dtype_name)
+    lr, rng = region(N, per, 0.5, 12)
+    tiles = sum(-(-w // 32) * -(-h // 2) for w, h in ((lr.isf[0], lr.isf[1]), (2 * N[0], 2 * N[1])))
+    most = 2 * torch.cuda.get_device_properties(0).multi_processor_count // tiles
+    assert most >= 1
+    pot = torch.tensor(rng.uniform(-1, 0, lr.nisf), dtype=dt, device="cuda")
+    one = torch.tensor(rng.uniform(-1, 1, lr.ncoeff), dtype=dt, device="cuda")
+    res = []
+    for norb in (most, most + 1):
+        b = Batch(wctx, [lr], [0] * norb)
+        h, ek, ep = b.locham(one.repeat(norb), pot)
+        assert torch.equal(h, h[:lr.ncoeff].repeat(norb))
+        res.append((h[:lr.ncoeff], ek[0].item(), ep[0].item()))
+    assert torch.equal(res[0][0], res[1][0])
+    for k in (1, 2):
+        assert abs(res[0][k] - res[1][k]) <= etol * abs(res[0][k])
