@@ -159,32 +159,10 @@ struct PlaneCells {
     }
 };
 
-// Scatter the compressed coefficients of wavelet plane kz into buffer A, which
-// must be zero.  psi points at [psi_c|psi_f]; sc (8 factors) scales each
-// component when non-null.
-template <class T, class TI, int S3>
-__device__ __forceinline__ void gather_plane_s(T *A, int pitch, const LrDev &L, int i3, const TI *psi, const T *sc)
-{
-    const PlaneCells p(L, pitch, i3, !S3);
-    const T s0 = sc ? sc[0] : T(1);
-    for_cells<8>(p.a_c + threadIdx.x, p.b_c, blockDim.x, L.pos_c, [&](int j, int at) { A[at] = (T)psi[j] * s0; });
-    const FineShare<S3> w;
-    const TI *pf = psi + L.nvctr_c - 1 + w.c;
-    T *a = A + comp_ofs(w.c, p.H1, p.wrow);
-    const T sf = sc ? sc[w.c] : T(1);
-    for_cells<8>(p.a_f + w.j0, w.in ? p.b_f : 0, w.step, L.pos_f, [&](int j, int at) { a[at] = (T)pf[7 * (size_t)j] * sf; });
-}
-
-// the z component s3 of a plane is uniform over the CTA: one copy of the
-// component loop per s3, so no instruction is issued for the other half
-template <class T, class TI>
-__device__ void gather_plane(T *A, int pitch, const LrDev &L, int kz, const TI *psi, const T *sc)
-{
-    if (kz >= L.N[2]) gather_plane_s<T, TI, 1>(A, pitch, L, kz - L.N[2], psi, sc);
-    else gather_plane_s<T, TI, 0>(A, pitch, L, kz, psi, sc);
-}
-
-// Inverse of gather_plane: write (or add into) the compressed output.
+// Write the wavelet plane kz into (or add it to) the compressed output at
+// [psi_c|psi_f]; sc (8 factors) scales each component when non-null.  The z
+// component s3 of a plane is uniform over the CTA: one copy of the component
+// loop per s3, so no instruction is issued for the other half.
 template <class T, class TO, int S3>
 __device__ __forceinline__ void scatter_plane_s(const T *A, int pitch, const LrDev &L, int i3, TO *out, bool accumulate,
                                                 const T *sc)
@@ -395,15 +373,17 @@ __device__ __forceinline__ void load_wavelet(T *B, int pitch, const Dims &d, con
     }
 }
 
-// gather_plane through cp.async (no scaling, same element type); the caller
-// waits.  Each coefficient is one queued copy to its slot of the plane.
+// Scatter the compressed coefficients of a wavelet plane (psi at [psi_c|psi_f])
+// into buffer A, which must be zero, through cp.async; the caller waits.  Each
+// coefficient is one queued copy to its slot of the plane.
 template <class T, int S3>
 __device__ __forceinline__ void gather_plane_async_s(T *A, int pitch, const LrDev &L, int i3, const T *psi)
 {
     const PlaneCells p(L, pitch, i3, !S3);
     for_cells<4>(p.a_c + threadIdx.x, p.b_c, blockDim.x, L.pos_c, [&](int j, int at) { cp_async_one(A + at, psi + j); });
     // a cell a lane here: the copies of a cell's values share its place and hit
-    // L1 after the first (values across lanes: K1 0.51 -> 0.57 ms on 128 x 48^3)
+    // L1 after the first (values across lanes: K1 0.51 -> 0.55 ms on 128 x 48^3,
+    // 0.33 -> 0.36 on 40^3)
     const T *pf = psi + L.nvctr_c;
     for_cells<4>(p.a_f + threadIdx.x, p.b_f, blockDim.x, L.pos_f, [&](int j, int at) {
         const T *src = pf + 7 * (size_t)j;
@@ -523,6 +503,7 @@ __device__ __forceinline__ void k1_item(const LrDev *__restrict__ lrs, const Orb
     extern __shared__ __align__(128) unsigned char smem_raw[];
     using U = typename ColUnit<T>::U;
     constexpr int kSeg = plane_seg(sizeof(T) == 4);
+    static_assert(std::is_same<T, TI>::value, "the gather copies elements as they are");
     {
         const int oi = find_owner(pre, norb, it);   // item = (orbital, wavelet plane kz)
         const int kz = it - pre[oi];
@@ -536,7 +517,7 @@ __device__ __forceinline__ void k1_item(const LrDev *__restrict__ lrs, const Orb
         if (MODE == MODE_PRECOND && threadIdx.x < 8) sc[threadIdx.x] = (T)prec_scal(L, cprec[oi], threadIdx.x);
         zero_region(A, d.G2, pitch);
         __syncthreads();
-        if (MODE == MODE_PRECOND && cg.dir && std::is_same<T, TI>::value) {
+        if (MODE == MODE_PRECOND && cg.dir) {
             // the CG direction, updated and scaled on the way in
             T *dv = cg.d + o.psi;
             const T *rv = cg.r + o.psi;
@@ -544,7 +525,7 @@ __device__ __forceinline__ void k1_item(const LrDev *__restrict__ lrs, const Orb
             const T beta = first ? T(0) : (T)(cg.rrn[oi] / cg.rr[oi]);
             if (kz >= d.N3) cg_dir_plane_s<T, 1>(A, pitch, L, kz - d.N3, dv, rv, beta, first, sc);
             else cg_dir_plane_s<T, 0>(A, pitch, L, kz, dv, rv, beta, first, sc);
-        } else if constexpr (std::is_same<T, TI>::value) {
+        } else {
             gather_plane_async<T>(A, pitch, L, kz, in_ptr(o, psi));
             cp_async_wait_all();
             if constexpr (MODE == MODE_PRECOND) {
@@ -555,8 +536,6 @@ __device__ __forceinline__ void k1_item(const LrDev *__restrict__ lrs, const Orb
                 for (int i = threadIdx.x; i < d.G2 * 2 * d.H1; i += blockDim.x, q.next())
                     A[q.r * pitch + q.c] *= sc[(q.c >= d.H1 ? 1 : 0) + (q.r >= d.N2 ? 2 : 0) + s3];
             }
-        } else {
-            gather_plane<T, TI>(A, pitch, L, kz, in_ptr(o, psi), MODE == MODE_PRECOND ? sc : nullptr);
         }
         __syncthreads();
         if (MODE != MODE_LOCDEN) store_wavelet(A, pitch, d, scratch + o.sP + (size_t)kz * d.G2 * d.G1);
@@ -610,7 +589,10 @@ __global__ void __launch_bounds__(NT, plane_min_blocks(sizeof(T) == 4, PERSIST, 
 // memory, chain 1 the tile alone; both write their outputs straight to global
 // memory, lanes on neighbouring columns.
 // At most NT threads per CTA (256, or for FP32 320 / 384), as many as share the
-// tile's segments evenly over its rounds (z_block).
+// tile's segments evenly over its rounds (z_block).  At the FP32 bounds of 256 and
+// 384 the compiler gives 80 registers and spills in chain 0 (64 bytes a thread
+// periodic, 112 free) and in free chain 1 (16 to 40); at 320 it gives 96 and
+// spills up to 16.
 __host__ __device__ constexpr int z_min_blocks(bool fp32, int nt) { return fp32 ? (nt > 256 ? 2 : 3) : 2; }
 
 template <class T, class TV, bool ALLPER, int CHAIN>

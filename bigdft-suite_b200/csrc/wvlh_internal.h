@@ -13,19 +13,26 @@ constexpr int TX_ = 32;
 constexpr int TY_ = 2;
 // Wavelet points of a line segment one thread takes in the fused kernels'
 // passes: eight, 16 accumulators in flight, as boxes are mostly multiples of
-// eight; six in the FP32 plane kernels, which then fill 384 threads on a 96 x 96
-// plane (K1 and K3 of 128 orbitals 0.51 + 1.19 ms, with eight 0.57 + 1.24).  The
-// FP64 plane kernels (32^3: K3 0.85 -> 0.68 ms) and the z kernel (40^3 FP32 0.60
-// -> 0.49 ms) gain from eight: fewer window loads an output.
+// eight; six in the FP32 plane kernels, whose passes then come in rounds that
+// divide better over their threads on most boxes (K1 + K3 of 128 orbitals, six
+// against eight points: 48^3 0.512 + 1.161 against 0.516 + 1.164 ms, 40^3 0.329 +
+// 0.780 against 0.336 + 0.824; 32^3 0.165 + 0.396 against 0.147 + 0.359 the other
+// way).  The FP64 plane kernels (32^3: K3 0.85 -> 0.68 ms) and the z kernel (40^3
+// FP32 0.60 -> 0.49 ms) gain from eight: fewer window loads an output.
 constexpr int kSegZ = 8;
 __host__ __device__ constexpr int plane_seg(bool fp32) { return fp32 ? 6 : 8; }
 // block size of the persistent plane kernels
 constexpr int kPlaneThreads = 384;
 
 // The plane kernels (K1, K3) run with any block size; they are compiled for
-// these bounds, at 65536 / (bound x CTAs per SM) registers a thread: FP32 56,
-// 56, 72, 64, 64; FP64 112, 168, 112, 112, 128.  Two planes of a 96 x 96 box
-// leave room for three FP32 CTAs or one FP64 CTA.
+// these bounds, at what the compiler gives a thread under bound x CTAs per SM:
+// FP32 56, 56, 72, 64, 64 registers; FP64 96, 168, 96, 96, 128 (576 threads are 18
+// warps, five to a quarter of the SM's registers).  K1 fits (at most 8 bytes
+// spilled), so does FP32 K3.  FP64 K3 spills 96 to 120 bytes a thread in periodic
+// and 264 to 324 in free boxes at 96 registers, 68 to 108 at 128, none at the
+// 384 bound; 576 threads still came out ahead of 384 (64 x 48^3: 2.46 against
+// 2.53 ms a call).  Two planes of a 96 x 96 box leave room for three FP32 CTAs or
+// one FP64 CTA.
 constexpr int kPlaneSizes[5] = {576, 384, 288, 192, 128};
 __host__ __device__ constexpr int plane_ctas_per_sm(bool fp32, int nt)
 {
@@ -151,7 +158,7 @@ struct Plan {
     // work items in runs of one orbital: prefix sums over the orbitals (norb+1
     // entries) of the plane kernels' items (G3 wavelet planes each) and of the
     // z kernels' 32 x 2-column tiles: chain 0 over I1 x I2 (d_pre2), chain 1
-    // over F1 x F2 (d_pre2p)
+    // over 2 N1 x 2 N2 (d_pre2p)
     int *d_pre13 = nullptr;
     int *d_pre2 = nullptr;
     int *d_pre2p = nullptr;
@@ -177,15 +184,16 @@ struct Plan {
     int part_stride = 0;           // energy partial slots per orbital
     size_t smem13[2] = {0, 0};     // dynamic smem bytes (float, double) of the two plane buffers
     long long plane_elems = 0;     // elements of plane buffer A (rows x pitch)
-    long long planeB_elems = 0;    // elements of buffer B (a plane or a transposed plane)
+    long long planeB_elems = 0;    // elements of buffer B (2 N2 rows)
     int plane_threads[2] = {kPlaneThreads, kPlaneThreads};   // plane-kernel CTA size (float, double)
     int plane_threads_pre[2] = {kPlaneThreads, kPlaneThreads};   // the same for the preconditioner operator
     int plane_cand[2][5] = {};                       // the sizes that the autotuner measures
     int z_segs0 = 1, z_segs1 = 1;                    // segments of the longest z line (chain 0, chain 1)
     int z_threads[2] = {kZThreads, kZThreads};       // z-kernel CTA bound (FP32: 256, 320 or 384)
     int z_threads_pre[2] = {kZThreads, kZThreads};   // the same for the preconditioner operator
+    // two tile columns of the longest grid in z: more than the z kernels ask for
+    // (smem_z0, smem_z1), it decides which boxes the entry points take
     size_t smem2[2] = {0, 0};
-    int pitch_max = 0, rows_max = 0, zlen_max = 0;
     size_t smem_z0[2] = {0, 0};    // dynamic smem bytes of the z kernel's chain 0 (and the density) ...
     size_t smem_z1[2] = {0, 0};    // ... and of chain 1
     // scratch elements per orbital when every orbital lies in one region (the

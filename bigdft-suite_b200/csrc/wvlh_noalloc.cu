@@ -6,7 +6,7 @@
 // library layers that must not grow the device footprint behind their host's
 // back.  For them this file gives one entry
 // point that runs the same fused kernels as wvlh_locham_batched, with every
-// table and all of its scratch (the P, Q/Z1 and Z2 planes and the energy
+// table and all of its scratch (the D, Q/Z1 and Z2 planes and the energy
 // partials) carved out of a file-scope static device array of fixed size.
 // The caller passes only its own inputs and outputs.
 #include <cuda_runtime.h>

@@ -69,8 +69,8 @@ struct wvlh_ctx {
 };
 
 // One localisation region: its box and its keys, validated once and kept on
-// the device in two forms: decoded {i0, i2, len, jj0} segments with per-plane
-// ranges (fused kernels) and the raw 1-based keys (one-pass-per-kernel path).
+// the device in two forms: cell tables with per-plane ranges (fused kernels)
+// and the raw 1-based keys (one-pass-per-kernel path).
 struct wvlh_region {
     int device = 0;
     wvlh::LrDev lr{};

@@ -544,7 +544,7 @@ int wvlh_locham_plain_batched(wvlh_batch *batch, const double *psi, const double
                               double *ekin, double *epot);
 
 /* CUDA graph of one wvlh_locham_batched call with fixed arguments (a packed
- * batch applied at every SCF iteration): the memsets and kernels are captured
+ * batch applied at every SCF iteration): the kernels are captured
  * once (on a private stream) and replayed by wvlh_graph_launch on the
  * context's stream with one launch.  The graph owns its scratch; the batch and
  * the buffers named at capture must outlive it.  Orbital batches are refused
