@@ -800,7 +800,8 @@ __global__ void __launch_bounds__(kZThreads, 2)
 }
 
 // ---------------------------------------------------------------------------
-// K3 (MODE_LOCHAM): Hpsi plane kz = B^T_x B^T_y Z1 + (T_x + T_y) D + Z2
+// K3 (MODE_LOCHAM): Hpsi plane kz = BInv6 B^T_x B^T_y Z1 + (T_x + T_y) D + Z2
+// (the FP32 taps of B are scaled)
 // K3 (MODE_PRECOND): D^-1/2 [(c + T_x + T_y) D + Z2]
 template <class T, class TO, bool ALLPER, int MODE>
 __device__ __forceinline__ void k3_item(const LrDev *__restrict__ lrs, const OrbDev *__restrict__ orbs,
